@@ -60,7 +60,57 @@ cudaError_t launch_set_scalar(double* p, double v, cudaStream_t s) {
 
 constexpr int SOR_NT = 1024;
 
+// The cluster kernel's shape for a grid, or V = 0 where sor_rb_kernel solves it:
+// the grid has to fit 16 CTAs of SOR_CL_MAXV pairs a thread (about 360^2,
+// beyond which the whole chip is as fast), a row the pairs of a CTA, and the
+// pairs the blocks of sor_rb_kernel one to a thread (an odd nx can exceed them
+// by a few), whose sums it repeats.
+struct SorClusterPlan { int V, nc; size_t smem; };
+static SorClusterPlan sor_cluster_plan(const SorArgs& a) {
+    SorClusterPlan p{0, 0, 0};
+    if (a.nx < 1 || a.ny < 1 || (long long)a.nx * a.ny > 2LL * SOR_CL_NT * SOR_CL_MAXV * SOR_CL_MAXC) return p;
+    if ((a.ax.periodic && (a.nx & 1)) || (a.ay.periodic && (a.ny & 1))) return p;
+    const int half = (a.nx + 1) / 2, M = half * a.ny;
+    const int nb = (M + SOR_NT - 1) / SOR_NT;
+    if (M > (a.nx * a.ny / 2 + SOR_NT - 1) / SOR_NT * SOR_NT) return p;
+    const int S = (nb + SOR_CL_MAXC - 1) / SOR_CL_MAXC * SOR_NT, V = S / SOR_CL_NT;
+    const size_t smem = sor_cluster_smem(S, half, nb);
+    if (V > SOR_CL_MAXV || half > S || smem > 224 * 1024) return p;
+    p.V = V; p.nc = (M + S - 1) / S; p.smem = smem;
+    return p;
+}
+
+template <int V> static cudaError_t launch_sor_cluster(const SorArgs& a, const SorClusterPlan& p, cudaStream_t s, bool* done) {
+    const void* fn = (const void*)sor_cluster_kernel<V>;
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    if (e == cudaSuccess && p.nc > 8) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = p.nc; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.nc); cfg.blockDim = dim3(SOR_CL_NT); cfg.dynamicSmemBytes = p.smem; cfg.stream = s;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    int clusters = 0;
+    e = cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg);
+    if (e != cudaSuccess || clusters < 1) { cudaGetLastError(); return cudaSuccess; }   // no room for such a cluster here
+    *done = true;
+    return cudaLaunchKernelEx(&cfg, sor_cluster_kernel<V>, a);
+}
+
 cudaError_t launch_sor(const SorArgs& a, int* nblocks_out, cudaStream_t s) {
+    const SorClusterPlan plan = sor_cluster_plan(a);
+    if (plan.V > 0) {
+        bool done = false;
+        cudaError_t ec = cudaSuccess;
+        switch (plan.V) {
+            case 2: ec = launch_sor_cluster<2>(a, plan, s, &done); break;
+            case 4: ec = launch_sor_cluster<4>(a, plan, s, &done); break;
+            case 6: ec = launch_sor_cluster<6>(a, plan, s, &done); break;
+            default: ec = launch_sor_cluster<8>(a, plan, s, &done); break;
+        }
+        if (ec != cudaSuccess || done) { if (nblocks_out) *nblocks_out = plan.nc; return ec; }
+    }
     int dev = 0, nsm = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;

@@ -17,6 +17,8 @@
 // removal after each sweep (applied lazily, see sor_rb_kernel), optional
 // residual test.
 #pragma once
+#include <cooperative_groups.h>
+
 #include "cc_device.cuh"
 
 namespace ccb {
@@ -442,6 +444,415 @@ __global__ void __launch_bounds__(NT) sor_rb_kernel(SorArgs a) {
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) { *a.iters_out = it; *a.res_out = res; }
+}
+
+// a / b for a b that many quotients share, correctly rounded (the double a / b
+// is): y = RN(1/b) once, then Markstein's correction steps (P. Markstein, IBM
+// J. Res. Dev. 34, 1990): q0 = a y is within two ulps, q1 = q0 + (a - b q0) y
+// is a faithful quotient, and from a faithful quotient the same step gives the
+// correctly rounded one.  Holds while nothing leaves the normal range, which
+// the exponent test of a guarantees for 2^-100 <= b <= 2^100 (ok_b); an
+// extreme a takes the division (a zero may: fast gives a zero too, sign aside).
+struct SharedDivisor {
+    double b, y;
+    bool ok_b;
+    __device__ __forceinline__ explicit SharedDivisor(double d) : b(d), y(1.0 / d) {
+        ok_b = d >= 0x1p-100 && d <= 0x1p100;
+    }
+    // the quotient where `inside(a)`, with no branch
+    __device__ __forceinline__ double fast(double a) const {
+        const double q0 = a * y;
+        const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+        return __fma_rn(__fma_rn(-b, q1, a), y, q1);
+    }
+    __device__ __forceinline__ bool inside(double a) const {   // 2^-895 <= |a| < 2^770
+        return ok_b && ((unsigned)__double2hiint(a) & 0x7fffffffu) - 0x08000000u <= 0x68000000u;
+    }
+    __device__ __forceinline__ double of(double a) const { return inside(a) ? fast(a) : a / b; }
+};
+
+// The same red-black SOR inside one thread-block cluster, for grids whose two
+// colours fit the shared memory of at most 16 CTAs (sor_cluster_plan).  What
+// bounds sor_rb_kernel on such grids is its grid barriers: 8.2 us a sweep at
+// 256^2 for under 1 us of FP64 work.  Here the potential never leaves the SMs
+// and CTAs exchange single values (st.async into the other CTA's shared
+// memory, counted by an mbarrier there), so that no phase waits for a fence:
+// a cluster barrier of 1024 threads takes 700 cycles with its release fence,
+// a counted store to a neighbour 260, to all of 16 CTAs 490.
+//
+// Cells go by pairs k = j half + p, the red and the black cell of columns 2p,
+// 2p + 1 of row j: N and S neighbours of either are the other colour's of
+// pairs k +- half, E and W those of k itself and of a pair next to it in the
+// row.  CTA c owns the pairs [c S, (c + 1) S), S >= half, and keeps both
+// colours on the window [c S - half, (c + 1) S + half); whoever updates a pair
+// stores it also into the windows of the CTAs that read it, the periodic
+// images of the first and last row included, so that every read is local.
+// A pair that reads another CTA's values is itself read by that CTA, so a
+// CTA's values of a phase can only arrive once every reader of the values
+// they replace has read (its own value, which depends on them, is awaited).
+// A thread keeps its V pairs and their right-hand sides in registers: a cell
+// takes three shared-memory loads instead of six, and the V cells' chains of
+// dependent FP64 operations overlap; 512 threads, for the registers (1024
+// threads of half as many pairs: 14.1 against 12.8 ms in the 256^2 MHD case).
+//
+// Measured, per sweep, sor_rb_kernel -> this: 32^2 6.5 -> 1.6 us, 128^2 6.7 ->
+// 2.1, 256^2 8.3 -> 3.4, 350^2 9.6 -> 7.2; with the residual test at 50^2
+// 10.7 -> 2.8.  V = 8 is the last that gains: ten pairs a thread (400^2) took
+// 10.2 us against 10.1.
+//
+// 1024 consecutive pairs are a block of sor_rb_kernel; S is a multiple of
+// 1024, and the field is summed by the same trees and in the same block order:
+// every double is that kernel's.
+constexpr int SOR_CL_NT = 512;
+constexpr int SOR_CL_MAXV = 8;      // pairs per thread
+constexpr int SOR_CL_MAXC = 16;     // CTAs of a cluster
+
+__host__ __device__ inline size_t sor_cluster_smem(int S, int half, int nb) {
+    return sizeof(double) * (2 * ((size_t)S + 2 * half) + (S / 32) * 33 + (S / 1024) * 33 + 2 * nb);
+}
+
+// sum of 32 doubles in the order of a shuffle-down tree (offsets 16, 8, 4, 2, 1)
+template <int O> __device__ __forceinline__ double tree32(const double* x, int l) {
+    if constexpr (O == 32) return x[l];
+    else return tree32<2 * O>(x, l) + tree32<2 * O>(x, l + O);
+}
+// the same by the four lanes q = 0 .. 3 of a group; every lane gets it
+__device__ __forceinline__ double tree32_by4(const double* x, int q) {
+    double r = tree32<4>(x, q);
+    r += __shfl_down_sync(0xffffffffu, r, 2);
+    r += __shfl_down_sync(0xffffffffu, r, 1);
+    return __shfl_sync(0xffffffffu, r, 0, 4);
+}
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned cluster_addr(unsigned local, int rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+    return r;
+}
+// store x at the shared-memory address `local` of CTA `rank` and count its 8 bytes on that CTA's mbarrier
+__device__ __forceinline__ void store_counted(unsigned local, unsigned mbar, int rank, double x) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
+                     cluster_addr(local, rank)),
+                 "l"(__double_as_longlong(x)), "r"(cluster_addr(mbar, rank))
+                 : "memory");
+}
+
+template <int V>
+__global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
+    if (a.active && *a.active == 0) return;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    constexpr int NT = SOR_CL_NT, S = V * NT;
+    static_assert(S % 1024 == 0, "whole blocks");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double s_val, s_res[SOR_CL_MAXC], s_max[NT / 32], s_over[2][SOR_CL_MAXC];
+    __shared__ __align__(8) unsigned long long s_bar[6];   // red, black, parts x 2, over x 2
+    const int nc = gridDim.x, c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nx = a.nx, ny = a.ny, half = (nx + 1) / 2, M = half * ny, W = S + 2 * half;
+    const int k0 = c * S, k1 = (k0 + S < M) ? k0 + S : M;
+    const int nb = (M + 1023) / 1024, N = nx * ny;
+    double* win = reinterpret_cast<double*>(smem_raw);   // red window (slot k - k0 + half), black window (+ W)
+    double* scr = win + 2 * W;                           // red + black of each own pair, 33 slots for 32
+    double* usum = scr + (S / 32) * 33;                  // sums of 32, 33 slots for the 32 of a block
+    double* parts = usum + (S / 1024) * 33;              // every block's sum, of this sweep and the last
+    const unsigned bars = smem_addr(s_bar), wins = smem_addr(win);
+    enum { RED = 0, BLACK = 8, PARTS = 16, OVER = 32 };
+    bool dead = false;
+    // wait for a phase of an mbarrier; bounded (about two seconds): a timeout is recorded and ends all further waits
+    auto wait = [&](unsigned bar, unsigned parity) {
+        if (dead) return;
+        long long t0 = 0;
+        for (int polls = 0;; polls++) {
+            unsigned ok = 0;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(ok)
+                : "r"(bars + bar), "r"(parity)
+                : "memory");
+            if (ok) return;
+            if ((polls & 1023) == 1023) {
+                if (t0 == 0) t0 = clock64();
+                else if (clock64() - t0 > (4ll << 30)) { atomicExch(a.bar.err, 1); dead = true; return; }
+            }
+        }
+    };
+    auto expect = [&](unsigned bar, unsigned bytes) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bars + bar), "r"(bytes) : "memory");
+    };
+    // bytes that other CTAs store into a window of this one in a phase (publish, below)
+    int halo = (c > 0 ? half : 0) + (c + 1 < nc ? (half < M - k1 ? half : M - k1) : 0);
+    if (a.ay.periodic) {
+        if (c > 0 && k1 + half > M) halo += k1 + half - M;
+        if (c == 0 && nc > 1) halo += half < M - S ? half : M - S;
+    }
+    const unsigned halo_bytes = 8u * halo, part_bytes = 8u * nb, over_bytes = 8u * nc;
+    if (tid == 0) {
+        for (int b = 0; b < 6; b++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8 * b) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // What a thread needs of its pairs, formed once: the window slots of the
+    // neighbours (16 bits each; .x: the x neighbour beside the pair for the red
+    // cell and for the black one, .y: N and S for the red cell, .z for the
+    // black one), bits of the pair and where other CTAs hold it (tgt: slot,
+    // rank << 16, SEND).  A clamped neighbour is the cell's own slot.
+    enum { HAS_R = 1, HAS_B = 2, CLAMPED = 4, ODD = 8, MANY = 16 };
+    constexpr unsigned SEND = 0x80000000u;
+    uint3 nbr[V];
+    unsigned tgt[V];
+    unsigned char st[V];
+    double vr[V], vb[V], hr[V], hb[V];
+    bool edge = false, sends = false;
+    // other windows that hold pair k: f(rank, slot in the red window)
+    auto holders = [&](int k, auto f) {
+        if (c > 0 && k < k0 + half) f(c - 1, k - (k0 - S) + half);
+        if (c + 1 < nc && k >= k0 + S - half) f(c + 1, k - (k0 + S) + half);
+        if (!a.ay.periodic) return;
+        if (k >= M - half) f(0, k - M + half);   // below row 0
+        if (k < half)                            // above the last row
+            for (int r = nc - 1; r >= 0 && r >= nc - 2; r--) {
+                const int end = ((r + 1) * S < M) ? (r + 1) * S : M;
+                if (k + M < end + half) f(r, k + M - r * S + half);
+            }
+    };
+    for (int q = tid; q < 2 * W; q += NT) win[q] = 0.0;
+    for (int q = tid; q < 2 * nb; q += NT) parts[q] = 0.0;
+    for (int q = tid; q < (S / 32) * 33 + (S / 1024) * 33; q += NT) scr[q] = 0.0;
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        const int own = v * NT + tid, k = k0 + own, me = own + half;
+        nbr[v] = make_uint3(0u, 0u, 0u);
+        tgt[v] = 0u;
+        st[v] = 0;
+        vr[v] = vb[v] = hr[v] = hb[v] = 0.0;
+        if (k >= k1) continue;
+        const int j = k / half, p = k - j * half, odd = j & 1;
+        const int ir = 2 * p + odd, ib = 2 * p + 1 - odd;
+        const bool perx = a.ax.periodic, pery = a.ay.periodic;
+        // A cell's x neighbours: the pair's other cell on one side (east of an even column, west of
+        // an odd one), a cell of the pair before or after on the other; a clamped one is the cell itself.
+        // slot of the one beside the pair, `oth` the offset of its colour's window
+        auto beside = [&](int i, int own_w, int oth) {
+            if (i & 1) return i + 1 < nx ? oth + me + 1 : (perx ? oth + me - half + 1 : own_w + me);
+            return i > 0 ? oth + me - 1 : (perx ? oth + me + half - 1 : own_w + me);
+        };
+        int f = odd ? ODD : 0;
+        if (ir < nx) f |= HAS_R;
+        if (ib < nx) f |= HAS_B;
+        // the last pair of an odd nx has one cell, an even column whose east neighbour is clamped
+        if ((!pery && (j == 0 || j + 1 == ny)) || (!perx && (ib == 0 || ib == nx - 1 || ir == 0 || ir == nx - 1))) f |= CLAMPED;
+        nbr[v].x = (unsigned)beside(ir, 0, W) | ((unsigned)beside(ib, W, 0) << 16);
+        const int up = (j + 1 < ny || pery) ? half : 0, down = (j > 0 || pery) ? half : 0;
+        nbr[v].y = (unsigned)(me + (up ? W + up : 0)) | ((unsigned)(me + (down ? W - down : 0)) << 16);
+        nbr[v].z = (unsigned)(me + (up ? up : W)) | ((unsigned)(me + (down ? -down : W)) << 16);
+        int holds = 0;
+        holders(k, [&](int rank, int slot) { tgt[v] = SEND | ((unsigned)rank << 16) | (unsigned)slot; holds++; });
+        if (holds > 1 || (holds == 1 && (int)((tgt[v] >> 16) & 0xff) == c)) f |= MANY;
+        edge |= holds > 0 && nc > 1;
+        sends |= holds > 0;
+        st[v] = (unsigned char)f;
+        if (ir < nx) hr[v] = a.rhs[(size_t)j * nx + ir];
+        if (ib < nx) hb[v] = a.rhs[(size_t)j * nx + ib];
+    }
+    edge = __any_sync(0xffffffffu, edge);   // the warp reads other CTAs' pairs
+    // store the value of the thread's pair v also where other CTAs (or the periodic images) read it
+    auto publish = [&](int v, int off, unsigned bar, double x) {   // off: 0 the red window, W the black one
+        if (!tgt[v]) return;
+        if (!(st[v] & MANY)) {
+            store_counted(wins + 8 * ((tgt[v] & 0xffffu) + off), bars + bar, (tgt[v] >> 16) & 0xff, x);
+            return;
+        }
+        holders(k0 + v * NT + tid, [&](int rank, int slot) {
+            if (rank == c) win[off + slot] = x;
+            else store_counted(wins + 8 * (off + slot), bars + bar, rank, x);
+        });
+    };
+    cl.sync();
+    const SharedDivisor denom(a.denom), cells((double)N);
+    const double omega = a.omega, idx2 = a.idx2, idy2 = a.idy2, tol = a.tol;
+    double m = 0.0;   // mean removal pending on every cell not yet rewritten in this sweep
+    double res = 0.0;
+    int it = 0;
+    // the neighbours W, E, N, S of the red (col 0) or black cell of pair v; `other`: the pair's other cell
+    auto gather = [&](int v, int col, double other, double& pW, double& pE, double& pN, double& pS) {
+        const unsigned y = col ? nbr[v].z : nbr[v].y;
+        const double b = win[col ? nbr[v].x >> 16 : nbr[v].x & 0xffffu];
+        // red cells of odd rows and black cells of even rows lie in odd columns
+        const bool oddcol = ((st[v] & ODD) != 0) != (col != 0);
+        pN = win[y & 0xffffu];
+        pS = win[y >> 16];
+        pW = oddcol ? other : b;
+        pE = oddcol ? b : other;
+    };
+    // whether the quotient a / denom needs the division (an extreme a; a zero does not)
+    auto extreme = [&](double q) {
+        return !denom.inside(q) && (__double2loint(q) | (__double2hiint(q) & 0x7fffffff)) != 0;
+    };
+    // max |lap(phi - m) - rhs| over the thread's cells
+    auto residual = [&]() {
+        double r = 0.0;
+#pragma unroll
+        for (int v = 0; v < V; v++) {
+#pragma unroll
+            for (int col = 0; col < 2; col++) {
+                if (!(st[v] & (col == 0 ? HAS_R : HAS_B))) continue;
+                double pW, pE, pN, pS;
+                gather(v, col, col == 0 ? vb[v] : vr[v], pW, pE, pN, pS);
+                const double x = (col == 0 ? vr[v] : vb[v]) - m;
+                pW -= m; pE -= m; pN -= m; pS -= m;
+                const double lap = (pE - 2.0 * x + pW) * idx2 + (pN - 2.0 * x + pS) * idy2;
+                r = fmax(r, fabs(lap - (col ? hb[v] : hr[v])));
+            }
+        }
+        return r;
+    };
+    // max over the cluster of the threads' r; every CTA gets it
+    auto cluster_max = [&](double r) {
+        for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_down_sync(0xffffffffu, r, o));
+        if (lane == 0) s_max[warp] = r;
+        __syncthreads();
+        if (tid == 0) {
+            for (int w = 1; w < NT / 32; w++) r = fmax(r, s_max[w]);
+            for (int q = 0; q < nc; q++) cl.map_shared_rank(s_res, q)[c] = r;
+        }
+        cl.sync();
+        double x = 0.0;
+        for (int q = 0; q < nc; q++) x = fmax(x, s_res[q]);
+        return x;
+    };
+    for (; it < a.max_iter; ++it) {
+        const unsigned ph = it & 1, ph2 = (it >> 1) & 1, two = 8 * (it & 1);
+        if (tid == 0) {
+            if (nc > 1) { expect(RED, halo_bytes); expect(BLACK, halo_bytes); }
+            expect(PARTS + two, part_bytes);
+        }
+        // Red: every value read is pending.  No branch but the rare ones, so that the V cells' chains
+        // overlap.  A cell that does not exist (odd nx) takes the value that its neighbour, whose
+        // clamped east it stands for, has there.
+        {
+            double q[V];
+            bool rare = false;
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                double pW, pE, pN, pS;
+                gather(v, 0, vb[v], pW, pE, pN, pS);
+                q[v] = ((pE - m) + (pW - m)) * idx2 + ((pN - m) + (pS - m)) * idy2 - hr[v];
+                rare |= extreme(q[v]);
+            }
+            if (rare) {
+#pragma unroll
+                for (int v = 0; v < V; v++) q[v] = q[v] / denom.b;
+            } else {
+#pragma unroll
+                for (int v = 0; v < V; v++) q[v] = denom.fast(q[v]);
+            }
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                const double x = vr[v] - m;
+                vr[v] = (st[v] & HAS_R) ? x + omega * (q[v] - x) : vb[v] - m;
+                if (st[v] & HAS_R) win[v * NT + tid + half] = vr[v];
+            }
+        }
+        if (sends) {
+#pragma unroll
+            for (int v = 0; v < V; v++) publish(v, 0, RED, vr[v]);
+        }
+        if (edge) wait(RED, ph);
+        __syncthreads();
+        // Black: the red neighbours are rewritten, a clamped one (the cell itself) is
+        // pending.  Sum every cell of the new field.
+        {
+            double q[V], x[V];
+            bool rare = false;
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                x[v] = vb[v] - m;
+                if (st[v] & CLAMPED) win[v * NT + tid + half + W] = x[v];   // read back as the clamped neighbour
+                double pW, pE, pN, pS;
+                gather(v, 1, vr[v], pW, pE, pN, pS);
+                q[v] = (pE + pW) * idx2 + (pN + pS) * idy2 - hb[v];
+                rare |= extreme(q[v]);
+            }
+            if (rare) {
+#pragma unroll
+                for (int v = 0; v < V; v++) q[v] = q[v] / denom.b;
+            } else {
+#pragma unroll
+                for (int v = 0; v < V; v++) q[v] = denom.fast(q[v]);
+            }
+#pragma unroll
+            for (int v = 0; v < V; v++) {
+                double s = 0.0;
+                if (st[v] & HAS_R) s += vr[v];
+                const double y = x[v] + omega * (q[v] - x[v]);
+                if (st[v] & HAS_B) s += y;
+                vb[v] = (st[v] & HAS_B) ? y : vr[v];
+                vr[v] = (st[v] & HAS_R) ? vr[v] : y;
+                if (st[v] & HAS_B) win[v * NT + tid + half + W] = y;
+                scr[(v * (NT / 32) + warp) * 33 + lane] = s;
+            }
+        }
+        if (sends) {
+#pragma unroll
+            for (int v = 0; v < V; v++) publish(v, W, BLACK, vb[v]);
+        }
+        __syncthreads();
+        // sums of 32 pairs by four lanes each, then the blocks' sums, to every CTA
+        const int q4 = tid & 3;
+#pragma unroll
+        for (int i = 0; i < (4 * S / 32 + NT - 1) / NT; i++) {
+            const int u = (i * NT + tid) >> 2;
+            if (4 * S / 32 % NT == 0 || u < S / 32) {   // whole warps
+                const double s = tree32_by4(scr + 33 * u, q4);
+                if (q4 == 0) usum[(u >> 5) * 33 + (u & 31)] = s;
+            }
+        }
+        __syncthreads();
+        double* pt = parts + (it & 1) * nb;
+        if (warp == 0) {
+            const int v = lane >> 2, b = c * (S / 1024) + v;
+            const double s = tree32_by4(usum + 33 * (v < S / 1024 ? v : 0), q4);
+            if (v < S / 1024 && b < nb)
+                for (int q = q4; q < nc; q += 4) store_counted(smem_addr(pt + b), bars + PARTS + two, q, s);
+            wait(PARTS + two, ph2);
+            if (lane == 0) {   // in block order
+                double t = 0.0;
+#pragma unroll 8
+                for (int q = 0; q < nb; q++) t += pt[q];
+                s_val = cells.of(t);
+            }
+        }
+        if (edge) wait(BLACK, ph);
+        __syncthreads();
+        m = s_val;
+        if (tol > 0.0) {
+            // the sweep's residual is needed only as "below tol or not", except after the last one
+            const double r = residual();
+            int any = __syncthreads_or(!(r < tol));
+            if (nc > 1) {
+                if (tid == 0) expect(OVER + two, over_bytes);
+                if (tid < nc) store_counted(smem_addr(&s_over[it & 1][c]), bars + OVER + two, tid, any ? 1.0 : 0.0);
+                wait(OVER + two, ph2);
+                any = 0;
+                for (int q = 0; q < nc; q++) any |= s_over[it & 1][q] != 0.0;
+            }
+            if (!any || it + 1 == a.max_iter) res = cluster_max(r);
+            if (!any) { ++it; break; }
+        }
+    }
+    if (!(tol > 0.0)) res = cluster_max(residual());
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        const int k = k0 + v * NT + tid;
+        if (k >= k1) continue;
+        const int j = k / half, p = k - j * half, odd = j & 1, ir = 2 * p + odd, ib = 2 * p + 1 - odd;
+        if (ir < nx) a.phi[(size_t)j * nx + ir] = vr[v] - m;
+        if (ib < nx) a.phi[(size_t)j * nx + ib] = vb[v] - m;
+    }
+    if (c == 0 && tid == 0) { *a.iters_out = it; *a.res_out = res; }
+    cl.sync();   // no CTA leaves while another may still store into its shared memory
 }
 
 // rhs = 4 pi G (rho - mean) (M2:187-194), mean from the density partial sums.
