@@ -95,12 +95,17 @@ cudaError_t M2Launch<T>::prepare(int nx, int ny) {
         }
     }
     constexpr int CW = (sizeof(T) == 8) ? 2 : 4;
-    const int smem_row = (int)(sizeof(Cplx<T>) * (size_t)fft_line_slots(nx));
-    const int smem_col = (int)(sizeof(Cplx<T>) * (size_t)fft_line_slots(ny) * CW);
+    const int smem_row = (int)(sizeof(Cplx<T>) * (size_t)fft_line_slots(nx)) * fft_lines_per_cta(nx, ny);
+    const int smem_col = (int)(sizeof(Cplx<T>) * (size_t)fft_col_stride(ny) * CW);
     if (smem_row <= 227 * 1024 && smem_col <= 227 * 1024) {  // larger lines are rejected by the solver set-up
-        CC_ATTR(fft_rows_fwd_kernel<T>, smem_row)
-        CC_ATTR(fft_rows_inv_kernel<T>, smem_row)
-        CC_ATTR((fft_cols_solve_kernel<T, CW>), smem_col)
+#define CC_FFT_ATTR(RB)                                          \
+        CC_ATTR((fft_rows_fwd_kernel<T, RB>), smem_row)          \
+        CC_ATTR((fft_rows_inv_kernel<T, RB>), smem_row)          \
+        CC_ATTR((fft_cols_solve_kernel<T, CW, RB>), smem_col)
+        CC_FFT_ATTR(2)
+        CC_FFT_ATTR(3)
+        CC_FFT_ATTR(4)
+#undef CC_FFT_ATTR
     }
 #undef CC_ATTR
     return cudaSuccess;
@@ -266,24 +271,42 @@ cudaError_t M2Launch<T>::pack_out_sum(const T* hi, const T* lo, double* dst, int
     return cudaGetLastError();
 }
 
+// Stages per pass of an n-point line of the FP64 transform.  Short lines leave
+// the SMs nearly empty, and fewer elements to a thread are more threads and
+// shorter chains; long lines fill them, and fewer passes win.  Column pass,
+// two / three / four stages: 128^2 6.0 / 8.3 / 11.8 us, 512^2 10.1 / 9.4 /
+// 19.1, 1024^2 32.0 / 31.4 / 27.2; the row passes turn at the same lengths.
+inline int fft_stages_per_pass(int n) { return n <= 256 ? 2 : (n <= 512 ? 3 : 4); }
+
 template <class T>
 cudaError_t M2Launch<T>::fft_solve(const T* rho, int pitch, const double* rho_part, int nx, int ny, int lognx,
                                    int logny, const Cplx<T>* twx_f, const Cplx<T>* twx_i, const Cplx<T>* twy_f,
                                    const Cplx<T>* twy_i, double Lx, double Ly, double G, Cplx<T>* A, T* phi,
                                    const int* active, cudaStream_t s) {
     constexpr int CW = (sizeof(T) == 8) ? 2 : 4;  // 32-byte column strips
-    const size_t smem_row = sizeof(Cplx<T>) * (size_t)fft_line_slots(nx);
-    const size_t smem_col = sizeof(Cplx<T>) * (size_t)fft_line_slots(ny) * CW;
+    const int rx = fft_stages_per_pass(nx), ry = fft_stages_per_pass(ny);
+    const int lines = fft_lines_per_cta(nx, ny), nt_row = fft_threads(nx, lines, rx);
+    const size_t smem_row = sizeof(Cplx<T>) * (size_t)fft_line_slots(nx) * lines;
+    const size_t smem_col = sizeof(Cplx<T>) * (size_t)fft_col_stride(ny) * CW;
+    const double ncell = (double)nx * (double)ny;
     cudaError_t e;
-    const int nt_row = nx >= 1024 ? 512 : (nx >= 256 ? 256 : 128);
-    fft_rows_fwd_kernel<T><<<ny, nt_row, smem_row, s>>>(rho, pitch, rho_part, RED_BLOCKS, (double)nx * (double)ny, A,
-                                                         nx, lognx, twx_f, active);
+#define CC_FFT_BY(R, LAUNCH) \
+    switch (R) {             \
+        case 2: { constexpr int RB = 2; LAUNCH; } break; \
+        case 3: { constexpr int RB = 3; LAUNCH; } break; \
+        default: { constexpr int RB = 4; LAUNCH; } break; \
+    }                        \
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    const int ncolblk = (nx + CW - 1) / CW;
-    fft_cols_solve_kernel<T, CW><<<ncolblk, 512, smem_col, s>>>(A, nx, ny, logny, twy_f, twy_i, Lx, Ly, G, active);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    fft_rows_inv_kernel<T><<<ny, nt_row, smem_row, s>>>(A, nx, lognx, twx_i, phi, pitch, active);
-    return cudaGetLastError();
+    CC_FFT_BY(rx, (fft_rows_fwd_kernel<T, RB><<<ny / lines, nt_row, smem_row, s>>>(
+                      rho, pitch, rho_part, RED_BLOCKS, ncell, A, nx, lognx, lines, twx_f, active)))
+    // one group of elements to a thread (fft_turn)
+    const int ncolblk = (nx + CW - 1) / CW, nt_col = fft_threads(ny, CW, ry);
+    CC_FFT_BY(ry, (fft_cols_solve_kernel<T, CW, RB><<<ncolblk, nt_col, smem_col, s>>>(A, nx, ny, logny, twy_f, twy_i, Lx,
+                                                                                      Ly, G, active)))
+    CC_FFT_BY(rx, (fft_rows_inv_kernel<T, RB><<<ny / lines, nt_row, smem_row, s>>>(A, nx, lognx, lines, twx_i, phi, pitch,
+                                                                                   active)))
+#undef CC_FFT_BY
+    return cudaSuccess;
 }
 
 template <class T>

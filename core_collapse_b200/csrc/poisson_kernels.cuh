@@ -18,6 +18,7 @@
 // residual test.
 #pragma once
 #include <cooperative_groups.h>
+#include <type_traits>
 
 #include "cc_device.cuh"
 
@@ -33,167 +34,291 @@ template <class T> __device__ __forceinline__ Cplx<T> cmul(Cplx<T> x, Cplx<T> w)
     return r;
 }
 
+// a / b for a b that many quotients share, correctly rounded (the double a / b
+// is): y = RN(1/b) once, then Markstein's correction steps (P. Markstein, IBM
+// J. Res. Dev. 34, 1990): q0 = a y is within two ulps, q1 = q0 + (a - b q0) y
+// is a faithful quotient, and from a faithful quotient the same step gives the
+// correctly rounded one.  Holds while nothing leaves the normal range, which
+// the exponent test of a guarantees for 2^-100 <= b <= 2^100 (ok_b); an
+// extreme a takes the division (a zero may: fast gives a zero too, sign aside).
+struct SharedDivisor {
+    double b, y;
+    bool ok_b;
+    __device__ __forceinline__ explicit SharedDivisor(double d) : b(d), y(1.0 / d) {
+        ok_b = d >= 0x1p-100 && d <= 0x1p100;
+    }
+    // the quotient where `inside(a)`, with no branch
+    __device__ __forceinline__ double fast(double a) const {
+        const double q0 = a * y;
+        const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+        return __fma_rn(__fma_rn(-b, q1, a), y, q1);
+    }
+    __device__ __forceinline__ bool inside(double a) const {   // 2^-895 <= |a| < 2^770
+        return ok_b && ((unsigned)__double2hiint(a) & 0x7fffffffu) - 0x08000000u <= 0x68000000u;
+    }
+    __device__ __forceinline__ double of(double a) const { return inside(a) ? fast(a) : a / b; }
+};
+
 __device__ __forceinline__ int bitrev(int i, int logn) { return (int)(__brev((unsigned)i) >> (32 - logn)); }
 
-// Shared-memory slot of element i of a transform line: one spare slot after
-// every 16, so that the strided accesses of the grouped passes below hit
+// Shared-memory slot of element i of a transform line: a spare slot after every
+// 16 and another after every 128, so that both the strided accesses of the
+// grouped passes below and the bit-reversed scatter of the first pass hit
 // distinct banks.  A line of n elements takes fft_line_slots(n) slots.
-__host__ __device__ constexpr int fft_line_slots(int n) { return n + (n >> 4); }
-__device__ __forceinline__ int fpad(int i) { return i + (i >> 4); }
+__host__ __device__ constexpr int fft_line_slots(int n) { return n + (n >> 4) + (n >> 7); }
+__device__ __forceinline__ int fpad(int i) { return i + (i >> 4) + (i >> 7); }
 
-// R consecutive radix-2 stages (half-lengths h0, 2 h0, ..., 2^(R-1) h0) of the
-// reference's DIT transform over `lines` lines of n elements in shared memory.
-// A thread takes the 2^R elements base + m h0 (m < 2^R) of one group, which
-// only exchange data among themselves in these stages, and runs the stages in
-// registers: every butterfly u = a[p], v = a[p+h] * tw[h-1 + (p mod h)],
-// a[p] = u + v, a[p+h] = u - v is the reference's, with the same operands and
-// twiddle, so the result is the same bit for bit as one stage per pass.
+// The transforms run R consecutive radix-2 stages of the reference's DIT
+// transform at a time (half-lengths h0, 2 h0, ..., 2^(R-1) h0): a thread takes
+// the 2^R elements base + m h0 (m < 2^R) of one group, which only exchange
+// data among themselves in these stages, and runs the stages in registers.
+// Every butterfly u = a[p], v = a[p+h] * tw[h-1 + (p mod h)], a[p] = u + v,
+// a[p+h] = u - v is the reference's, with the same operands and twiddle, so the
+// result is the same bit for bit as one stage per pass.
+//
+// These kernels are bound by latency (a line of 1024 points is three passes),
+// so a CTA has the threads that its groups need and no more: eight CTAs of 64
+// threads to an SM at n = 1024 where 512 threads, 448 of them waiting, held it
+// alone.  The first pass takes its elements from the loads (the group of
+// thread g after bit reversal is elements g, g + n/2^R, ...: coalesced), the
+// last one hands its results to the stores, and between the forward and the
+// inverse column transform they stay in registers: four trips through shared
+// memory to a column instead of nine.  FP64 solve (rows, columns, inverse
+// rows), before -> now: 128^2 20.7 -> 14.2 us, 512^2 49 -> 20, 1024^2 148 ->
+// 49, 2048^2 403 -> 188.
 template <class T, int R>
-__device__ __forceinline__ void fft_group_pass(Cplx<T>* a, int n, int lines, int h0,
-                                               const Cplx<T>* __restrict__ tw) {
+__device__ __forceinline__ void fft_stages(Cplx<T> (&x)[1 << R], int h0, int o, const Cplx<T>* __restrict__ tw) {
     constexpr int M = 1 << R;
-    const int gpl = n >> R;   // groups per line
-    const int L = fft_line_slots(n);
+#pragma unroll
+    for (int st = 0; st < R; st++) {
+        const int hs = 1 << st, h = h0 << st;
+#pragma unroll
+        for (int m = 0; m < M; m++) {
+            if (m & hs) continue;
+            const Cplx<T> w = tw[h - 1 + o + (m & (hs - 1)) * h0];   // p mod h = o + (m mod hs) h0
+            const Cplx<T> u = x[m];
+            const Cplx<T> v = cmul(x[m + hs], w);
+            x[m].re = u.re + v.re; x[m].im = u.im + v.im;
+            x[m + hs].re = u.re - v.re; x[m + hs].im = u.im - v.im;
+        }
+    }
+}
+
+// m with its R bits reversed
+template <int R> __host__ __device__ constexpr int rev_bits(int m) {
+    int r = 0;
+    for (int b = 0; b < R; b++) r |= ((m >> b) & 1) << (R - 1 - b);
+    return r;
+}
+
+// work item g of `lines` lines with gpl groups each: line l, group q.  IL: the
+// lines interleaved (adjacent columns in adjacent threads).
+template <bool IL> __device__ __forceinline__ void fft_item(int g, int lines, int gpl, int& l, int& q) {
+    if (IL) { l = g % lines; q = g / lines; }
+    else { l = g / gpl; q = g - l * gpl; }
+}
+
+// First stages (h0 = 1): elements from ld(line, natural index), results to the
+// lines in shared memory, or to st(line, index, x) where n = 2^R (LAST).
+template <class T, int R, bool IL, bool LAST, class LD, class ST>
+__device__ __forceinline__ void fft_first(Cplx<T>* a, int LS, int n, int logn, int lines, const Cplx<T>* __restrict__ tw, LD ld,
+                                          ST st) {
+    constexpr int M = 1 << R;
+    const int gpl = n >> R;
     for (int g = threadIdx.x; g < lines * gpl; g += blockDim.x) {
-        const int l = g / gpl, gg = g - l * gpl;
-        const int o = gg & (h0 - 1), blk = gg / h0;
-        Cplx<T>* line = a + l * L;
-        const int base = blk * (M * h0) + o;
+        int l, q;
+        fft_item<IL>(g, lines, gpl, l, q);
+        Cplx<T> x[M];
+#pragma unroll
+        for (int m = 0; m < M; m++) x[m] = ld(l, rev_bits<R>(m) * gpl + q);
+        fft_stages<T, R>(x, 1, 0, tw);
+        const int base = (LAST ? 0 : bitrev(q, logn - R)) * M;
+#pragma unroll
+        for (int m = 0; m < M; m++) {
+            if (LAST) st(l, base + m, x[m]);
+            else a[l * LS + fpad(base + m)] = x[m];
+        }
+    }
+    __syncthreads();
+}
+
+// Stages h0 .. 8 h0 within shared memory, or out of it through st(line, index, x) (LAST, 16 h0 = n).
+template <class T, int R, bool IL, bool LAST, class ST>
+__device__ __forceinline__ void fft_next(Cplx<T>* a, int LS, int n, int lines, int h0, const Cplx<T>* __restrict__ tw, ST st) {
+    constexpr int M = 1 << R;
+    const int gpl = n >> R;
+    for (int g = threadIdx.x; g < lines * gpl; g += blockDim.x) {
+        int l, q;
+        fft_item<IL>(g, lines, gpl, l, q);
+        const int o = q & (h0 - 1), base = (q / h0) * (M * h0) + o;
+        Cplx<T>* line = a + l * LS;
         Cplx<T> x[M];
 #pragma unroll
         for (int m = 0; m < M; m++) x[m] = line[fpad(base + m * h0)];
+        fft_stages<T, R>(x, h0, o, tw);
 #pragma unroll
-        for (int st = 0; st < R; st++) {
-            const int hs = 1 << st, h = h0 << st;
-#pragma unroll
-            for (int m = 0; m < M; m++) {
-                if (m & hs) continue;
-                const Cplx<T> w = tw[h - 1 + o + (m & (hs - 1)) * h0];   // p mod h = o + (m mod hs) h0
-                const Cplx<T> u = x[m];
-                const Cplx<T> v = cmul(x[m + hs], w);
-                x[m].re = u.re + v.re; x[m].im = u.im + v.im;
-                x[m + hs].re = u.re - v.re; x[m + hs].im = u.im - v.im;
-            }
+        for (int m = 0; m < M; m++) {
+            if (LAST) st(l, base + m * h0, x[m]);
+            else line[fpad(base + m * h0)] = x[m];
         }
-#pragma unroll
-        for (int m = 0; m < M; m++) line[fpad(base + m * h0)] = x[m];
     }
     __syncthreads();
 }
 
-// All log2(n) stages over `lines` lines already in bit-reversed order (line l
-// at a + l fft_line_slots(n), padded slots), four stages per pass.
-// tw: twiddles of all stages, half-length h at tw[h-1 .. 2h-2].
-template <class T>
-__device__ __forceinline__ void fft_passes(Cplx<T>* a, int n, int lines, const Cplx<T>* __restrict__ tw) {
-    int h0 = 1;
-    while (h0 < n) {
-        const int left = n / h0;
-        if (left >= 16) { fft_group_pass<T, 4>(a, n, lines, h0, tw); h0 <<= 4; }
-        else if (left == 8) { fft_group_pass<T, 3>(a, n, lines, h0, tw); h0 <<= 3; }
-        else if (left == 4) { fft_group_pass<T, 2>(a, n, lines, h0, tw); h0 <<= 2; }
-        else { fft_group_pass<T, 1>(a, n, lines, h0, tw); h0 <<= 1; }
-    }
+// f(std::integral_constant<int, r>) for 1 <= r <= RB
+template <int RB, class F> __device__ __forceinline__ void with_radix(int r, F f) {
+    if constexpr (RB >= 4)
+        if (r == 4) { f(std::integral_constant<int, 4>()); return; }
+    if constexpr (RB >= 3)
+        if (r == 3) { f(std::integral_constant<int, 3>()); return; }
+    if (r == 2) f(std::integral_constant<int, 2>());
+    else f(std::integral_constant<int, 1>());
 }
 
-// the three kernels below run on at most FFT_NT threads
+// A whole transform of `lines` lines, RB stages a pass; the first pass takes what logn leaves over.
+// tw: twiddles of all stages, half-length h at tw[h-1 .. 2h-2].
+template <class T, int RB, bool IL, class LD, class ST>
+__device__ __forceinline__ void fft_lines(Cplx<T>* a, int LS, int n, int logn, int lines, const Cplx<T>* __restrict__ tw,
+                                          LD ld, ST st) {
+    const int r = (logn - 1) % RB + 1;
+    if (r == logn) {
+        with_radix<RB>(r, [&](auto R) { fft_first<T, decltype(R)::value, IL, true>(a, LS, n, logn, lines, tw, ld, st); });
+        return;
+    }
+    with_radix<RB>(r, [&](auto R) { fft_first<T, decltype(R)::value, IL, false>(a, LS, n, logn, lines, tw, ld, st); });
+    int h0 = 1 << r;
+    for (; (h0 << RB) < n; h0 <<= RB) fft_next<T, RB, IL, false>(a, LS, n, lines, h0, tw, st);
+    fft_next<T, RB, IL, true>(a, LS, n, lines, h0, tw, st);
+}
+
+// the kernels below run on at most FFT_NT threads
 constexpr int FFT_NT = 512;
 
-// pass 1: one block per row.  rho is a pitched T field; mean = sum/N.
-template <class T>
+// lines of an n-point transform to a CTA (of `total`), and its threads: one per group of 16
+__host__ __device__ inline int fft_lines_per_cta(int n, int total) {
+    const int l = n >= 512 ? 1 : 512 / n;
+    return l < total ? l : total;
+}
+__host__ __device__ inline int fft_threads(int n, int lines, int RB) {
+    const int t = ((lines * n >> RB) + 31) / 32 * 32;
+    return t < 32 ? 32 : (t > FFT_NT ? FFT_NT : t);
+}
+
+// the mean of a density whose partial sums are given, by the CTA's first warp
+__device__ __forceinline__ double fft_mean(const double* __restrict__ rho_part, int nparts, double ncell, double* sh) {
+    if (threadIdx.x < 32) {
+        double s = 0.0;
+        for (int b = threadIdx.x; b < nparts; b += 32) s += rho_part[b];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (threadIdx.x == 0) *sh = s / ncell;
+    }
+    __syncthreads();
+    return *sh;
+}
+
+// pass 1: `lines` rows per block.  rho is a pitched T field; mean = sum/N.
+template <class T, int RB>
 __global__ void __launch_bounds__(FFT_NT) fft_rows_fwd_kernel(const T* __restrict__ rho, int pitch, const double* __restrict__ rho_part,
-                                    int nparts, double ncell, Cplx<T>* __restrict__ A, int nx, int logn,
+                                    int nparts, double ncell, Cplx<T>* __restrict__ A, int nx, int logn, int lines,
                                     const Cplx<T>* __restrict__ tw, const int* __restrict__ active) {
     if (active && *active == 0) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Cplx<T>* a = reinterpret_cast<Cplx<T>*>(smem_raw);
     __shared__ double s_mean;
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int b = 0; b < nparts; b++) s += rho_part[b];
-        s_mean = s / ncell;
-    }
-    __syncthreads();
-    const T mean = (T)s_mean;
-    const int j = blockIdx.x;
-    for (int i = threadIdx.x; i < nx; i += blockDim.x) {
-        Cplx<T> z;
-        z.re = rho[(size_t)j * pitch + i] - mean;
-        z.im = T(0);
-        a[fpad(bitrev(i, logn))] = z;
-    }
-    __syncthreads();
-    fft_passes(a, nx, 1, tw);
-    for (int i = threadIdx.x; i < nx; i += blockDim.x) A[(size_t)j * nx + i] = a[fpad(i)];
+    const T mean = (T)fft_mean(rho_part, nparts, ncell, &s_mean);
+    const size_t j0 = (size_t)blockIdx.x * lines;
+    fft_lines<T, RB, false>(reinterpret_cast<Cplx<T>*>(smem_raw), fft_line_slots(nx), nx, logn, lines, tw,
+        [&](int l, int i) { return Cplx<T>{rho[(j0 + l) * pitch + i] - mean, T(0)}; },
+        [&](int l, int i, Cplx<T> z) { A[(j0 + l) * nx + i] = z; });
 }
+
+// The spectral factor K(k) = -4 pi G / |k|^2 (NS:308-322, continuous |k|^2,
+// zero mode removed) between the forward and the inverse transform of a
+// column.  The last forward pass and the first inverse one have the same radix
+// 2^H, so that a thread's elements q + m n/2^H stay in its registers (one group
+// to a thread).  ONLY: they are the whole transforms (n = 2^H), from ld to st.
+template <class T, int H, int CW, bool ONLY, class LD, class ST>
+__device__ __forceinline__ void fft_turn(Cplx<T>* a, int LS, int n, int logn, double kx, double Ly, double fourpiG,
+                                         const Cplx<T>* __restrict__ twf, const Cplx<T>* __restrict__ twi, LD ld, ST st) {
+    constexpr int M = 1 << H;
+    const int gpl = n >> H, l = threadIdx.x % CW, q = threadIdx.x / CW;
+    const bool mine = q < gpl;
+    const SharedDivisor by_Ly(Ly);
+    const double two_pi = 2.0 * M_PI;
+    Cplx<T> y[M];
+    if (mine) {
+        Cplx<T> x[M];
+#pragma unroll
+        for (int m = 0; m < M; m++) x[m] = ONLY ? ld(l, rev_bits<H>(m)) : a[l * LS + fpad(q + m * gpl)];
+        fft_stages<T, H>(x, gpl, q, twf);
+#pragma unroll
+        for (int m = 0; m < M; m++) {
+            const int j = q + m * gpl, nj = (j <= n / 2) ? j : j - n;
+            const double ky = by_Ly.of(two_pi * (double)nj);
+            const double k2 = kx * kx + ky * ky;
+            const T f = (k2 == 0.0) ? T(0) : (T)(-fourpiG / k2);
+            // the inverse's first pass takes element rev(m) n/2^H + q as its m-th
+            y[rev_bits<H>(m)] = Cplx<T>{x[m].re * f, x[m].im * f};
+        }
+        fft_stages<T, H>(y, 1, 0, twi);
+    }
+    __syncthreads();   // every element of the forward transform is read
+    if (mine) {
+        const int base = (ONLY ? 0 : bitrev(q, logn - H)) * M;
+#pragma unroll
+        for (int m = 0; m < M; m++) {
+            if (ONLY) st(l, m, y[m]);
+            else a[l * LS + fpad(base + m)] = y[m];
+        }
+    }
+    __syncthreads();
+}
+
+// line stride of the interleaved columns: half a bank row off, so that the two columns of adjacent
+// threads hit distinct banks
+__host__ __device__ inline int fft_col_stride(int n) { return (fft_line_slots(n) + 7) / 8 * 8 + 4; }
 
 // pass 2: CW adjacent columns per block: forward FFT along y, spectral
 // multiply, inverse FFT along y.
-template <class T, int CW>
+template <class T, int CW, int RB>
 __global__ void __launch_bounds__(FFT_NT) fft_cols_solve_kernel(Cplx<T>* __restrict__ A, int nx, int ny, int logn,
                                       const Cplx<T>* __restrict__ twf, const Cplx<T>* __restrict__ twi,
                                       double Lx, double Ly, double G, const int* __restrict__ active) {
     if (active && *active == 0) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Cplx<T>* a = reinterpret_cast<Cplx<T>*>(smem_raw);   // CW padded lines of ny
-    const int L = fft_line_slots(ny);
-    const int c0 = blockIdx.x * CW;
-    for (int k = threadIdx.x; k < CW * ny; k += blockDim.x) {
-        const int cc = k % CW, j = k / CW;
-        a[cc * L + fpad(bitrev(j, logn))] = A[(size_t)j * nx + c0 + cc];
+    const int LS = fft_col_stride(ny), c0 = blockIdx.x * CW, i = c0 + (int)threadIdx.x % CW;
+    const double kx = 2.0 * M_PI * (double)((i <= nx / 2) ? i : i - nx) / Lx, fourpiG = 4.0 * M_PI * G;
+    const T inv = T(1.0) / (T)ny;   // ny is a power of two: z * inv is z / ny
+    auto ld = [&](int l, int j) { return A[(size_t)j * nx + c0 + l]; };
+    auto st = [&](int l, int j, Cplx<T> z) { A[(size_t)j * nx + c0 + l] = Cplx<T>{z.re * inv, z.im * inv}; };
+    auto none = [](int, int, Cplx<T>) {};
+    const int r = (logn - 1) % RB + 1;
+    if (r == logn) {
+        with_radix<RB>(r, [&](auto R) {
+            fft_turn<T, decltype(R)::value, CW, true>(a, LS, ny, logn, kx, Ly, fourpiG, twf, twi, ld, st);
+        });
+        return;
     }
-    __syncthreads();
-    fft_passes(a, ny, CW, twf);
-    // spectral kernel (NS:308-322), continuous |k|^2, zero mode removed
-    const double two_pi = 2.0 * M_PI;
-    for (int k = threadIdx.x; k < CW * ny; k += blockDim.x) {
-        const int cc = k % CW, j = k / CW, i = c0 + cc;
-        const int nj = (j <= ny / 2) ? j : j - ny;
-        const int ni = (i <= nx / 2) ? i : i - nx;
-        const double ky = two_pi * (double)nj / Ly;
-        const double kx = two_pi * (double)ni / Lx;
-        const double k2 = kx * kx + ky * ky;
-        Cplx<T>& z = a[cc * L + fpad(j)];
-        if (k2 == 0.0) { z.re = T(0); z.im = T(0); }
-        else {
-            const T s = (T)(-(4.0 * M_PI * G) / k2);
-            z.re = z.re * s; z.im = z.im * s;
-        }
-    }
-    __syncthreads();
-    // bit-reverse permutation of each line for the inverse DIT transform
-    for (int k = threadIdx.x; k < CW * ny; k += blockDim.x) {
-        const int cc = k / ny, j = k % ny, r = bitrev(j, logn);
-        if (j < r) {
-            Cplx<T> t = a[cc * L + fpad(j)];
-            a[cc * L + fpad(j)] = a[cc * L + fpad(r)];
-            a[cc * L + fpad(r)] = t;
-        }
-    }
-    __syncthreads();
-    fft_passes(a, ny, CW, twi);
-    const T n = (T)ny;
-    for (int k = threadIdx.x; k < CW * ny; k += blockDim.x) {
-        const int cc = k % CW, j = k / CW;
-        Cplx<T> z = a[cc * L + fpad(j)];
-        z.re = z.re / n; z.im = z.im / n;
-        A[(size_t)j * nx + c0 + cc] = z;
-    }
+    with_radix<RB>(r, [&](auto R) { fft_first<T, decltype(R)::value, true, false>(a, LS, ny, logn, CW, twf, ld, none); });
+    for (int h0 = 1 << r; (h0 << RB) < ny; h0 <<= RB) fft_next<T, RB, true, false>(a, LS, ny, CW, h0, twf, none);
+    fft_turn<T, RB, CW, false>(a, LS, ny, logn, kx, Ly, fourpiG, twf, twi, ld, st);
+    int h0 = 1 << RB;
+    for (; (h0 << r) < ny; h0 <<= RB) fft_next<T, RB, true, false>(a, LS, ny, CW, h0, twi, none);
+    with_radix<RB>(r, [&](auto R) { fft_next<T, decltype(R)::value, true, true>(a, LS, ny, CW, h0, twi, st); });
 }
 
-// pass 3: inverse FFT along x, real part -> phi (pitched).
-template <class T>
-__global__ void __launch_bounds__(FFT_NT) fft_rows_inv_kernel(const Cplx<T>* __restrict__ A, int nx, int logn, const Cplx<T>* __restrict__ tw,
-                                    T* __restrict__ phi, int pitch, const int* __restrict__ active) {
+// pass 3: inverse FFT along x, real part -> phi (pitched), `lines` rows per block.
+template <class T, int RB>
+__global__ void __launch_bounds__(FFT_NT) fft_rows_inv_kernel(const Cplx<T>* __restrict__ A, int nx, int logn, int lines,
+                                    const Cplx<T>* __restrict__ tw, T* __restrict__ phi, int pitch,
+                                    const int* __restrict__ active) {
     if (active && *active == 0) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Cplx<T>* a = reinterpret_cast<Cplx<T>*>(smem_raw);
-    const int j = blockIdx.x;
-    for (int i = threadIdx.x; i < nx; i += blockDim.x) a[fpad(bitrev(i, logn))] = A[(size_t)j * nx + i];
-    __syncthreads();
-    fft_passes(a, nx, 1, tw);
-    const T n = (T)nx;
-    for (int i = threadIdx.x; i < nx; i += blockDim.x) phi[(size_t)j * pitch + i] = a[fpad(i)].re / n;
+    const size_t j0 = (size_t)blockIdx.x * lines;
+    const T inv = T(1.0) / (T)nx;   // nx is a power of two: x * inv is x / nx
+    fft_lines<T, RB, false>(reinterpret_cast<Cplx<T>*>(smem_raw), fft_line_slots(nx), nx, logn, lines, tw,
+        [&](int l, int i) { return A[(j0 + l) * nx + i]; },
+        [&](int l, int i, Cplx<T> z) { phi[(j0 + l) * pitch + i] = z.re * inv; });
 }
 
 // ---------------------------------------------------------------------------
@@ -445,31 +570,6 @@ __global__ void __launch_bounds__(NT) sor_rb_kernel(SorArgs a) {
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) { *a.iters_out = it; *a.res_out = res; }
 }
-
-// a / b for a b that many quotients share, correctly rounded (the double a / b
-// is): y = RN(1/b) once, then Markstein's correction steps (P. Markstein, IBM
-// J. Res. Dev. 34, 1990): q0 = a y is within two ulps, q1 = q0 + (a - b q0) y
-// is a faithful quotient, and from a faithful quotient the same step gives the
-// correctly rounded one.  Holds while nothing leaves the normal range, which
-// the exponent test of a guarantees for 2^-100 <= b <= 2^100 (ok_b); an
-// extreme a takes the division (a zero may: fast gives a zero too, sign aside).
-struct SharedDivisor {
-    double b, y;
-    bool ok_b;
-    __device__ __forceinline__ explicit SharedDivisor(double d) : b(d), y(1.0 / d) {
-        ok_b = d >= 0x1p-100 && d <= 0x1p100;
-    }
-    // the quotient where `inside(a)`, with no branch
-    __device__ __forceinline__ double fast(double a) const {
-        const double q0 = a * y;
-        const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
-        return __fma_rn(__fma_rn(-b, q1, a), y, q1);
-    }
-    __device__ __forceinline__ bool inside(double a) const {   // 2^-895 <= |a| < 2^770
-        return ok_b && ((unsigned)__double2hiint(a) & 0x7fffffffu) - 0x08000000u <= 0x68000000u;
-    }
-    __device__ __forceinline__ double of(double a) const { return inside(a) ? fast(a) : a / b; }
-};
 
 // The same red-black SOR inside one thread-block cluster, for grids whose two
 // colours fit the shared memory of at most 16 CTAs (sor_cluster_plan).  What
