@@ -21,6 +21,106 @@ template <class T> __host__ __device__ constexpr T tiny_pos() { return sizeof(T)
 __host__ __device__ __forceinline__ int wrap_idx(int i, int n) { int r = i % n; return (r < 0) ? r + n : r; }
 __host__ __device__ __forceinline__ int clamp_idx(int i, int lo, int hi) { return i < lo ? lo : (i > hi ? hi : i); }
 
+// Correctly rounded FP64 quotients without a branch.  A division is 13
+// operations on the FP64 pipe and ends in a branch to its slow path, so that
+// one waits for the other: a chain of 120 cycles each (107 cycles of a warp's
+// issue instead of 27 when the numerator is a zero, which the velocity and
+// field components that a planar flow does not have are).  The forms below
+// overlap, and quotients of one denominator share its reciprocal.
+//   y = RN(1/b): the hardware's approximation, one third-order Newton step (an
+//   error below 2^-59 before its rounding, so y is within one ulp), and one step
+//   that rounds it correctly, unless b's significand is all ones.
+//   a / b from y: q0 = a y is within two ulps, q1 = q0 + (a - b q0) y is a
+//   faithful quotient, and from a faithful quotient the same step gives RN(a/b).
+// Both last steps are Markstein's (P. Markstein, Computation of elementary
+// functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990).
+// They hold while nothing leaves the normal range: divisor_inside and
+// quotient_inside; what they refuse, a caller divides.
+__device__ __forceinline__ double recip_fast(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = __fma_rn(-b, y, 1.0);
+    y = __fma_rn(y, __fma_rn(e, e, e), y);
+    return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+}
+__device__ __forceinline__ double quotient_fast(double a, double b, double y) {
+    const double q0 = a * y;
+    const double q1 = __fma_rn(-__fma_rn(b, q0, -a), y, q0);
+    return __fma_rn(-__fma_rn(b, q1, -a), y, q1);
+}
+__device__ __forceinline__ bool divisor_inside(double b) {    // 2^-100 <= |b| < 2^101, significand not all ones
+    const unsigned hi = (unsigned)__double2hiint(b);
+    return (hi & 0x7fffffffu) - 0x39b00000u < 0x0c900000u && ((hi | 0xfff00000u) & (unsigned)__double2loint(b)) != ~0u;
+}
+__device__ __forceinline__ bool quotient_inside(double a) {   // a zero, or 2^-895 <= |a| < 2^770
+    const unsigned hi = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    return hi - 0x08000000u <= 0x68000000u || (hi | (unsigned)__double2loint(a)) == 0u;
+}
+// a / b with y = RN(1/b) at hand (by a zero the sign of the zero may be the other one for b < 0)
+__device__ __forceinline__ double quotient(double a, double b, double y) {
+    return divisor_inside(b) && quotient_inside(a) ? quotient_fast(a, b, y) : a / b;
+}
+
+// The divisions of a pointwise function in type T.  FP32: one reciprocal per
+// shared denominator and products with it.  FP64: the host and PLAIN divide; the
+// device forms quotients by the functions above and sets `rare` where one of
+// them is outside their range: the caller then evaluates the function again
+// with PLAIN.  So every FP64 result is the divisions' own.
+template <class T, bool PLAIN> struct Div {
+    bool rare = false;
+#if defined(__CUDA_ARCH__)
+    static constexpr bool FAST64 = sizeof(T) == 8 && !PLAIN;
+#else
+    static constexpr bool FAST64 = false;
+#endif
+    // what quot takes beside the denominator b
+    __host__ __device__ __forceinline__ T recip(T b) {
+#if defined(__CUDA_ARCH__)
+        if constexpr (FAST64) {
+            rare |= !divisor_inside(b);
+            return recip_fast(b);
+        }
+#endif
+        if constexpr (sizeof(T) == 4) return T(1.0) / b;
+        else return T(0.0);
+    }
+    __host__ __device__ __forceinline__ T quot(T a, T b, T y) {
+#if defined(__CUDA_ARCH__)
+        if constexpr (FAST64) {
+            rare |= !quotient_inside(a);
+            return quotient_fast(a, b, y);
+        }
+#endif
+        if constexpr (sizeof(T) == 4) return a * y;
+        else return a / b;
+    }
+    // the same with a reciprocal that the host has rounded (constants of the grid)
+    __host__ __device__ __forceinline__ T quot_by(T a, T b, T y) {
+#if defined(__CUDA_ARCH__)
+        if constexpr (FAST64) rare |= !divisor_inside(b);
+#endif
+        return quot(a, b, y);
+    }
+    // a / b, a denominator of its own
+    __host__ __device__ __forceinline__ T div(T a, T b) {
+        if constexpr (FAST64) return quot(a, b, recip(b));
+        else return a / b;
+    }
+};
+
+// f(d) with the fast divisions, again with the plain ones where they do not apply
+template <class T, class F> __host__ __device__ __forceinline__ auto divided(F f) {
+    Div<T, false> d;
+    auto r = f(d);
+    if constexpr (Div<T, false>::FAST64) {
+        if (d.rare) {
+            Div<T, true> p;
+            r = f(p);
+        }
+    }
+    return r;
+}
+
 // One grid axis.  Cell indices wrap modulo n (periodic) or clamp to [0,n-1];
 // face indices along the axis wrap modulo n+1 or clamp to [0,n]
 // (mhd2d_resistive_hlld_ct_gravity.cpp:241-252).

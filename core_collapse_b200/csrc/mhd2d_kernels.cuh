@@ -101,12 +101,15 @@ __device__ __forceinline__ void joule_terms(const M2Const<T>& c, const Fields<T>
     const int jN = c.ay.cell(j + 1), jS = c.ay.cell(j - 1);
     const T bzE = s.Bz[(size_t)j * P + iE], bzW = s.Bz[(size_t)j * P + iW];
     const T bzN = s.Bz[(size_t)jN * P + i], bzS = s.Bz[(size_t)jS * P + i];
-    const T dBzdy = div_or_mul(bzN - bzS, c.two_dy, T(0.5) * c.inv_dy);
-    const T dBzdx = div_or_mul(bzE - bzW, c.two_dx, T(0.5) * c.inv_dx);
-    const T dBydx = div_or_mul(s.by[(size_t)j * P + iE] - s.by[(size_t)j * P + i], c.dx, c.inv_dx);
-    const T dBxdy = div_or_mul(s.bx[(size_t)jN * P + i] - s.bx[(size_t)j * P + i], c.dy, c.inv_dy);
-    const T Jx = dBzdy, Jy = -dBzdx, Jz = dBydx - dBxdy;
-    J2 = Jx * Jx + Jy * Jy + Jz * Jz;
+    const T dby = s.by[(size_t)j * P + iE] - s.by[(size_t)j * P + i], dbx = s.bx[(size_t)jN * P + i] - s.bx[(size_t)j * P + i];
+    J2 = divided<T>([&](auto& d) {
+        const T dBzdy = d.quot_by(bzN - bzS, c.two_dy, T(0.5) * c.inv_dy);
+        const T dBzdx = d.quot_by(bzE - bzW, c.two_dx, T(0.5) * c.inv_dx);
+        const T dBydx = d.quot_by(dby, c.dx, c.inv_dx);
+        const T dBxdy = d.quot_by(dbx, c.dy, c.inv_dy);
+        const T Jx = dBzdy, Jy = -dBzdx, Jz = dBydx - dBxdy;
+        return Jx * Jx + Jy * Jy + Jz * Jz;
+    });
     lap = (bzE - T(2) * bzC + bzW) * c.idx2 + (bzN - T(2) * bzC + bzS) * c.idy2;
 }
 
@@ -405,9 +408,13 @@ __device__ __forceinline__ void m2_stage_tile(const M2Const<T>& c, const Fields<
         if (c.resistive) {
             const int ci = c.ax.cell(ie), cim = c.ax.cell(ie - 1);
             const int cj = c.ay.cell(je), cjm = c.ay.cell(je - 1);
-            const T dBydx = div_or_mul(in.by[(size_t)je * P + ci] - in.by[(size_t)je * P + cim], c.dx, c.inv_dx);
-            const T dBxdy = div_or_mul(in.bx[(size_t)cj * P + ie] - in.bx[(size_t)cjm * P + ie], c.dy, c.inv_dy);
-            res = c.eta * (dBydx - dBxdy);
+            const T dby = in.by[(size_t)je * P + ci] - in.by[(size_t)je * P + cim];
+            const T dbx = in.bx[(size_t)cj * P + ie] - in.bx[(size_t)cjm * P + ie];
+            res = divided<T>([&](auto& d) {
+                const T dBydx = d.quot_by(dby, c.dx, c.inv_dx);
+                const T dBxdy = d.quot_by(dbx, c.dy, c.inv_dy);
+                return c.eta * (dBydx - dBxdy);
+            });
         }
         ez[k] = ideal + res;
     }
@@ -458,7 +465,13 @@ __device__ __forceinline__ void m2_stage_tile(const M2Const<T>& c, const Fields<
         }
     }
     // CT (M2:807-830) for this cell's four faces
-    const T dtdy = dt / c.dy, dtdx = dt / c.dx;
+    T dtdy, dtdx;
+    if constexpr (fast_recip<T>()) {
+        dtdy = dt / c.dy; dtdx = dt / c.dx;
+    } else {
+        dtdy = divided<T>([&](auto& d) { return d.quot_by(dt, c.dy, c.inv_dy); });
+        dtdx = divided<T>([&](auto& d) { return d.quot_by(dt, c.dx, c.inv_dx); });
+    }
     const T e00 = ez[ty * (TX + 1) + tx], e10 = ez[ty * (TX + 1) + tx + 1];
     const T e01 = ez[(ty + 1) * (TX + 1) + tx], e11 = ez[(ty + 1) * (TX + 1) + tx + 1];
     T bxL, bxR, byD, byU;
@@ -493,17 +506,13 @@ __device__ __forceinline__ void m2_stage_tile(const M2Const<T>& c, const Fields<
             const T* phi = ga;
             const int iE = c.ax.cell(gi + 1), iW = c.ax.cell(gi - 1);
             const int jN = c.ay.cell(gj + 1), jS = c.ay.cell(gj - 1);
-            gxq = div_or_mul(-(phi[(size_t)gj * P + iE] - phi[(size_t)gj * P + iW]), c.two_dx, T(0.5) * c.inv_dx);
-            gyq = div_or_mul(-(phi[(size_t)jN * P + gi] - phi[(size_t)jS * P + gi]), c.two_dy, T(0.5) * c.inv_dy);
+            const T px = -(phi[(size_t)gj * P + iE] - phi[(size_t)gj * P + iW]);
+            const T py = -(phi[(size_t)jN * P + gi] - phi[(size_t)jS * P + gi]);
+            gxq = divided<T>([&](auto& d) { return d.quot_by(px, c.two_dx, T(0.5) * c.inv_dx); });
+            gyq = divided<T>([&](auto& d) { return d.quot_by(py, c.two_dy, T(0.5) * c.inv_dy); });
         }
-        T u, v;
-        if constexpr (fast_recip<T>()) {
-            const T ir = T(1.0) / vmax(rho, tiny_pos<T>());
-            u = mx * ir; v = my * ir;
-        } else {
-            u = mx / vmax(rho, tiny_pos<T>());
-            v = my / vmax(rho, tiny_pos<T>());
-        }
+        const Vel<T> V = velocity(vmax(rho, tiny_pos<T>()), mx, my, T(0.0));
+        const T u = V.u, v = V.v;
         if constexpr (KAHAN) {
             comp_add(mx, lmx, dt * rho * gxq);
             comp_add(my, lmy, dt * rho * gyq);

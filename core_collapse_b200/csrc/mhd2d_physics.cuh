@@ -41,7 +41,13 @@ __host__ __device__ __forceinline__ Prim<T> prim_select(bool left, const Prim<T>
 // The FP32 bulk path is issue-bound and each of its divisions is several
 // instructions, so where one denominator serves several quotients it takes
 // one reciprocal and multiplies (a rounding change of an ulp); FP64 keeps the
-// reference's divisions operation for operation.
+// reference's quotients, each rounded as its division rounds it, but forms them
+// without the division's branch (Div in cc_device.cuh): the stage kernel is
+// bound by chains of dependent operations at 20 warps an SM, and the divisions
+// were the longest.  1024^2 stage kernel, second stage: 323 -> 255 us, RK
+// average 73 -> 55; 3D faces at 90 x 70 x 52 with the hybrid equation of state
+// 57 -> 50.  Sharing reciprocals alone, with a branch to each quotient, gained
+// nothing (328 us).
 template <class T> __host__ __device__ constexpr bool fast_recip() { return sizeof(T) == 4; }
 
 // 1/b on the fast-reciprocal path, else 0 (never read there): the FP64 build
@@ -57,17 +63,21 @@ template <class T> __host__ __device__ __forceinline__ T div_or_mul(T a, T b, T 
     else return a / b;
 }
 
+template <class T> struct Vel { T u, v, w; };
+// (mx, my, mz) / rho
+template <class T> __host__ __device__ __forceinline__ Vel<T> velocity(T rho, T mx, T my, T mz) {
+    return divided<T>([&](auto& d) {
+        const T ir = d.recip(rho);
+        return Vel<T>{d.quot(mx, rho, ir), d.quot(my, rho, ir), d.quot(mz, rho, ir)};
+    });
+}
+
 // enforce_floors (M2:114-124)
 template <class T>
 __host__ __device__ __forceinline__ void floors(const M2Const<T>& c, T& rho, T mx, T my, T mz, T& E, T Bx, T By, T Bz) {
     rho = vmax(rho, c.floor_rho);
-    T u, v, w;
-    if constexpr (fast_recip<T>()) {
-        const T ir = T(1.0) / rho;
-        u = mx * ir; v = my * ir; w = mz * ir;
-    } else {
-        u = mx / rho; v = my / rho; w = mz / rho;
-    }
+    const Vel<T> V = velocity(rho, mx, my, mz);
+    const T u = V.u, v = V.v, w = V.w;
     T kin = T(0.5) * rho * (u * u + v * v + w * w);
     T mag = T(0.5) * (Bx * Bx + By * By + Bz * Bz);
     T P = c.gm1 * (E - kin - mag);
@@ -81,13 +91,8 @@ __host__ __device__ __forceinline__ void floors(const M2Const<T>& c, T& rho, T m
 template <class T>
 __host__ __device__ __forceinline__ Prim<T> to_prim(const M2Const<T>& c, T rho, T mx, T my, T mz, T E, T Bx, T By, T Bz) {
     rho = vmax(rho, c.floor_rho);
-    T u, v, w;
-    if constexpr (fast_recip<T>()) {
-        const T ir = T(1.0) / rho;
-        u = mx * ir; v = my * ir; w = mz * ir;
-    } else {
-        u = mx / rho; v = my / rho; w = mz / rho;
-    }
+    const Vel<T> V = velocity(rho, mx, my, mz);
+    const T u = V.u, v = V.v, w = V.w;
     T kin = T(0.5) * rho * (u * u + v * v + w * w);
     T mag = T(0.5) * (Bx * Bx + By * By + Bz * Bz);
     T P = c.gm1 * (E - kin - mag);
@@ -97,19 +102,24 @@ __host__ __device__ __forceinline__ Prim<T> to_prim(const M2Const<T>& c, T rho, 
     return W;
 }
 
+// What the energy and the speeds of a state share beyond the state: nothing
+// for the ideal gas (the cold part of the pressure in 3D, mhd3d_physics.cuh).
+struct NoEos {};
+template <class T> __host__ __device__ __forceinline__ NoEos eos_of(const M2Const<T>&, const Prim<T>&) { return {}; }
+
 // total energy of a primitive state, ideal gas (M2:357, 397, 482, 495)
-template <class T>
-__host__ __device__ __forceinline__ T energy(const M2Const<T>& c, const Prim<T>& W) {
+template <class T, class D>
+__host__ __device__ __forceinline__ T energy(const M2Const<T>& c, const Prim<T>& W, NoEos, D& d) {
     T B2 = W.bx * W.bx + W.by * W.by + W.bz * W.bz;
     T eint;
     if constexpr (fast_recip<T>()) eint = W.P * (T(1.0) / c.gm1);   // 1/gm1 shared by every call in a face
-    else eint = W.P / c.gm1;
+    else eint = d.quot(W.P, c.gm1, d.recip(c.gm1));
     return eint + T(0.5) * W.r * (W.u * W.u + W.v * W.v + W.w * W.w) + T(0.5) * B2;
 }
 
 // fast magnetosonic speed with normal component bn (M2:148-174)
-template <class T>
-__host__ __device__ __forceinline__ T fast_speed(const M2Const<T>& c, const Prim<T>& W, T bn) {
+template <class T, class D>
+__host__ __device__ __forceinline__ T fast_speed(const M2Const<T>& c, const Prim<T>& W, T bn, NoEos, D& d) {
     T b2 = W.bx * W.bx + W.by * W.by + W.bz * W.bz;
     T a2, vA2, vn2;
     if constexpr (fast_recip<T>()) {
@@ -121,15 +131,27 @@ __host__ __device__ __forceinline__ T fast_speed(const M2Const<T>& c, const Prim
         vA2 = b2 * ir;
         vn2 = (bn * bn) * ir;
     } else {
-        a2 = c.gamma * W.P / vmax(W.r, c.floor_rho);
-        const T rho = vmax(W.r, tiny_pos<T>());
-        vA2 = b2 / rho;
-        vn2 = (bn * bn) / rho;
+        const T rf = vmax(W.r, c.floor_rho), rho = vmax(W.r, tiny_pos<T>());
+        const T ir = d.recip(rho);
+        a2 = (rf == rho) ? d.quot(c.gamma * W.P, rho, ir) : c.gamma * W.P / rf;
+        vA2 = d.quot(b2, rho, ir);
+        vn2 = d.quot(bn * bn, rho, ir);
     }
     T disc = (a2 + vA2) * (a2 + vA2) - T(4.0) * a2 * vn2;
     disc = vmax(T(0.0), disc);
     T cf2 = T(0.5) * ((a2 + vA2) + sqrt(disc));
     return sqrt(vmax(T(0.0), cf2));
+}
+
+template <class T, class Cst> __host__ __device__ __forceinline__ T energy_of(const Cst& c, const Prim<T>& W) {
+    return divided<T>([&](auto& d) { return energy(c, W, eos_of(c, W), d); });
+}
+template <class T, class Cst> __host__ __device__ __forceinline__ T fast_speed_of(const Cst& c, const Prim<T>& W, T bn) {
+    return divided<T>([&](auto& d) { return fast_speed(c, W, bn, eos_of(c, W), d); });
+}
+template <class T> __host__ __device__ __forceinline__ T energy(const M2Const<T>& c, const Prim<T>& W) { return energy_of(c, W); }
+template <class T> __host__ __device__ __forceinline__ T fast_speed(const M2Const<T>& c, const Prim<T>& W, T bn) {
+    return fast_speed_of(c, W, bn);
 }
 
 // x-normal ideal flux (M2:351-370; M3:396-413 with the hybrid-EOS energy).
@@ -173,21 +195,32 @@ __host__ __device__ __forceinline__ Flux<T> ideal_flux_ep(const Prim<T>& W, T E,
 // HLLD (M2:372-530), the reference's own star / double-star construction:
 // degenerate guards at 1e-14, HLL fallback for |Bn| < 1e-12, double-star
 // fluxes jumped from the outer state with the outer speed.
-template <class T, class Cst>
-__host__ __device__ __forceinline__ Flux<T> hlld_x_scalar(const Cst& c, Prim<T> L, Prim<T> R, T Bn) {
+template <class T, class Cst, class D>
+__host__ __device__ __forceinline__ Flux<T> hlld_x_by(const Cst& c, Prim<T> L, Prim<T> R, T Bn, D& d) {
     L.bx = Bn; R.bx = Bn;
-    const T cfL = fast_speed(c, L, Bn), cfR = fast_speed(c, R, Bn);
+    const auto xL = eos_of(c, L), xR = eos_of(c, R);
+    const T cfL = fast_speed(c, L, Bn, xL, d), cfR = fast_speed(c, R, Bn, xR, d);
     const T SL = vmin(L.u - cfL, R.u - cfR);
     const T SR = vmax(L.u + cfL, R.u + cfR);
-    if (T(0.0) <= SL) return ideal_flux(c, L);
-    if (T(0.0) >= SR) return ideal_flux(c, R);
+    // FP32 forms the energy of a flux again (ideal_flux), which keeps its rounding the same in every
+    // kernel that inlines this (the batched tile shapes give bit-identical results)
+    if (T(0.0) <= SL) {
+        if constexpr (fast_recip<T>()) return ideal_flux(c, L);
+        else return ideal_flux_ep(L, energy(c, L, xL, d), L.P + T(0.5) * (L.bx * L.bx + L.by * L.by + L.bz * L.bz));
+    }
+    if (T(0.0) >= SR) {
+        if constexpr (fast_recip<T>()) return ideal_flux(c, R);
+        else return ideal_flux_ep(R, energy(c, R, xR, d), R.P + T(0.5) * (R.bx * R.bx + R.by * R.by + R.bz * R.bz));
+    }
 
-    const T EL = energy(c, L), ER = energy(c, R);
+    const T EL = energy(c, L, xL, d), ER = energy(c, R, xR, d);
     const T ptL = L.P + T(0.5) * (L.bx * L.bx + L.by * L.by + L.bz * L.bz);
     const T ptR = R.P + T(0.5) * (R.bx * R.bx + R.by * R.by + R.bz * R.bz);
 
     if (fabs(Bn) < T(1e-12)) {  // HLL (M2:449-467)
-        const Flux<T> FL = ideal_flux(c, L), FR = ideal_flux(c, R);
+        Flux<T> FL, FR;
+        if constexpr (fast_recip<T>()) { FL = ideal_flux(c, L); FR = ideal_flux(c, R); }
+        else { FL = ideal_flux_ep(L, EL, ptL); FR = ideal_flux_ep(R, ER, ptR); }
         const T inv = T(1.0) / (SR - SL);
         const T s2 = SL * SR;
         Flux<T> F;
@@ -203,10 +236,17 @@ __host__ __device__ __forceinline__ Flux<T> hlld_x_scalar(const Cst& c, Prim<T> 
 
     const T den = L.r * (SL - L.u) - R.r * (SR - R.u);
     T SM = T(0.0);
-    if (fabs(den) > T(1e-14)) SM = (ptR - ptL + L.r * L.u * (SL - L.u) - R.r * R.u * (SR - R.u)) / den;
+    if (fabs(den) > T(1e-14)) SM = d.div(ptR - ptL + L.r * L.u * (SL - L.u) - R.r * R.u * (SR - R.u), den);
 
-    const T rLs = L.r * (SL - L.u) / (SL - SM);
-    const T rRs = R.r * (SR - R.u) / (SR - SM);
+    const T iSL = d.recip(SL - SM), iSR = d.recip(SR - SM);
+    T rLs, rRs;
+    if constexpr (fast_recip<T>()) {
+        rLs = L.r * (SL - L.u) / (SL - SM);
+        rRs = R.r * (SR - R.u) / (SR - SM);
+    } else {
+        rLs = d.quot(L.r * (SL - L.u), SL - SM, iSL);
+        rRs = d.quot(R.r * (SR - R.u), SR - SM, iSR);
+    }
     const T pts = ptL + L.r * (SL - L.u) * (SM - L.u);
     const T sL = SL - L.u, sR = SR - R.u;
     const T bn2 = Bn * Bn;
@@ -225,10 +265,11 @@ __host__ __device__ __forceinline__ Flux<T> hlld_x_scalar(const Cst& c, Prim<T> 
             vLs = L.v - (ByLs - L.by) * bq;
             wLs = L.w - (BzLs - L.bz) * bq;
         } else {
-            ByLs = L.by * num / dL;
-            BzLs = L.bz * num / dL;
-            vLs = L.v - Bn * (ByLs - L.by) / dd;
-            wLs = L.w - Bn * (BzLs - L.bz) / dd;
+            const T id = d.recip(dL), idd = d.recip(dd);
+            ByLs = d.quot(L.by * num, dL, id);
+            BzLs = d.quot(L.bz * num, dL, id);
+            vLs = L.v - d.quot(Bn * (ByLs - L.by), dd, idd);
+            wLs = L.w - d.quot(Bn * (BzLs - L.bz), dd, idd);
         }
     }
     if (fabs(dR) > T(1e-14)) {
@@ -241,10 +282,11 @@ __host__ __device__ __forceinline__ Flux<T> hlld_x_scalar(const Cst& c, Prim<T> 
             vRs = R.v - (ByRs - R.by) * bq;
             wRs = R.w - (BzRs - R.bz) * bq;
         } else {
-            ByRs = R.by * num / dR;
-            BzRs = R.bz * num / dR;
-            vRs = R.v - Bn * (ByRs - R.by) / dd;
-            wRs = R.w - Bn * (BzRs - R.bz) / dd;
+            const T id = d.recip(dR), idd = d.recip(dd);
+            ByRs = d.quot(R.by * num, dR, id);
+            BzRs = d.quot(R.bz * num, dR, id);
+            vRs = R.v - d.quot(Bn * (ByRs - R.by), dd, idd);
+            wRs = R.w - d.quot(Bn * (BzRs - R.bz), dd, idd);
         }
     }
     T sqL, sqR, SLL, SRR;
@@ -260,8 +302,8 @@ __host__ __device__ __forceinline__ Flux<T> hlld_x_scalar(const Cst& c, Prim<T> 
     } else {
         sqL = sqrt(vmax(rLs, tiny_pos<T>()));
         sqR = sqrt(vmax(rRs, tiny_pos<T>()));
-        SLL = SM - fabs(Bn) / sqL;
-        SRR = SM + fabs(Bn) / sqR;
+        SLL = SM - d.div(fabs(Bn), sqL);
+        SRR = SM + d.div(fabs(Bn), sqR);
     }
 
     // pick the region first, then build only the state it needs
@@ -285,19 +327,19 @@ __host__ __device__ __forceinline__ Flux<T> hlld_x_scalar(const Cst& c, Prim<T> 
             Bys = (sqL * ByRs + sqR * ByLs + sqL * sqR * (vRs - vLs) * sgn) * id2;
             Bzs = (sqL * BzRs + sqR * BzLs + sqL * sqR * (wRs - wLs) * sgn) * id2;
         } else {
-            vs = (sqL * vLs + sqR * vRs + (ByRs - ByLs) * sgn) / d2;
-            ws = (sqL * wLs + sqR * wRs + (BzRs - BzLs) * sgn) / d2;
-            Bys = (sqL * ByRs + sqR * ByLs + sqL * sqR * (vRs - vLs) * sgn) / d2;
-            Bzs = (sqL * BzRs + sqR * BzLs + sqL * sqR * (wRs - wLs) * sgn) / d2;
+            const T id2 = d.recip(d2);
+            vs = d.quot(sqL * vLs + sqR * vRs + (ByRs - ByLs) * sgn, d2, id2);
+            ws = d.quot(sqL * wLs + sqR * wRs + (BzRs - BzLs) * sgn, d2, id2);
+            Bys = d.quot(sqL * ByRs + sqR * ByLs + sqL * sqR * (vRs - vLs) * sgn, d2, id2);
+            Bzs = d.quot(sqL * BzRs + sqR * BzLs + sqL * sqR * (wRs - wLs) * sgn, d2, id2);
         }
     }
     // U_star (M2:486-505) and the jump F_W + S (U* - U_W) (M2:507-519)
     const T vBs = SM * Bn + vs * Bys + ws * Bzs;
     const T vBw = W.u * W.bx + W.v * W.by + W.w * W.bz;
-    const T Es = ((S - W.u) * EW - (ptW * W.u - Bn * vBw) + (pts * SM - Bn * vBs)) / (S - SM);
-    // FP64: the flux from the known energy and total pressure (the same values);
-    // FP32 forms them again, which keeps its rounding the same in every kernel
-    // that inlines this (the batched tile shapes give bit-identical results)
+    T Es;
+    if constexpr (fast_recip<T>()) Es = ((S - W.u) * EW - (ptW * W.u - Bn * vBw) + (pts * SM - Bn * vBs)) / (S - SM);
+    else Es = d.quot((S - W.u) * EW - (ptW * W.u - Bn * vBw) + (pts * SM - Bn * vBs), S - SM, left ? iSL : iSR);
     Flux<T> F;
     if constexpr (fast_recip<T>()) F = ideal_flux(c, W);
     else F = ideal_flux_ep(W, EW, ptW);
@@ -308,6 +350,26 @@ __host__ __device__ __forceinline__ Flux<T> hlld_x_scalar(const Cst& c, Prim<T> 
     F.f4 = F.f4 + S * (Es - EW);
     F.f5 = F.f5 + S * (Bys - W.by);
     F.f6 = F.f6 + S * (Bzs - W.bz);
+    return F;
+}
+
+// the face again with plain divisions (Div), out of line
+template <class T, class Cst> __host__ __device__ __noinline__ void hlld_x_plain(const Cst& c, const Prim<T>& L, const Prim<T>& R, T Bn, Flux<T>& F) {
+    Div<T, true> p;
+    F = hlld_x_by(c, L, R, Bn, p);
+}
+template <class T, class Cst>
+__host__ __device__ __forceinline__ Flux<T> hlld_x_scalar(const Cst& c, const Prim<T>& L, const Prim<T>& R, T Bn) {
+    Div<T, false> d;
+    Flux<T> F = hlld_x_by(c, L, R, Bn, d);
+    if constexpr (Div<T, false>::FAST64) {
+        if (d.rare) {
+            const Prim<T> l = L, r = R;
+            Flux<T> f;
+            hlld_x_plain(c, l, r, Bn, f);
+            F = f;
+        }
+    }
     return F;
 }
 

@@ -493,9 +493,11 @@ __global__ void __launch_bounds__(256) m3_emf_ct_kernel(const M3Const<T> c, cons
 // CFL speeds of a cell in three directions (compute_dt loop body, M3:633-636)
 template <class T>
 __device__ __forceinline__ double speed3(const M3Const<T>& c, const Prim<T>& W) {
-    const T sx = fabs(W.u) + fast_speed(c, W, W.bx);
-    const T sy = fabs(W.v) + fast_speed(c, W, W.by);
-    const T sz = fabs(W.w) + fast_speed(c, W, W.bz);
+    const ColdEos<T> cd = eos_of(c, W);
+    auto cf = [&](T bn) { return divided<T>([&](auto& d) { return fast_speed(c, W, bn, cd, d); }); };
+    const T sx = fabs(W.u) + cf(W.bx);
+    const T sy = fabs(W.v) + cf(W.by);
+    const T sz = fabs(W.w) + cf(W.bz);
     // std::max(maxs, x) ignores NaN x; keep each finite value
     double m = 0.0;
     if ((double)sx > m) m = (double)sx;

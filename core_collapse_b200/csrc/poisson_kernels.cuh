@@ -34,31 +34,6 @@ template <class T> __device__ __forceinline__ Cplx<T> cmul(Cplx<T> x, Cplx<T> w)
     return r;
 }
 
-// a / b for a b that many quotients share, correctly rounded (the double a / b
-// is): y = RN(1/b) once, then Markstein's correction steps (P. Markstein, IBM
-// J. Res. Dev. 34, 1990): q0 = a y is within two ulps, q1 = q0 + (a - b q0) y
-// is a faithful quotient, and from a faithful quotient the same step gives the
-// correctly rounded one.  Holds while nothing leaves the normal range, which
-// the exponent test of a guarantees for 2^-100 <= b <= 2^100 (ok_b); an
-// extreme a takes the division (a zero may: fast gives a zero too, sign aside).
-struct SharedDivisor {
-    double b, y;
-    bool ok_b;
-    __device__ __forceinline__ explicit SharedDivisor(double d) : b(d), y(1.0 / d) {
-        ok_b = d >= 0x1p-100 && d <= 0x1p100;
-    }
-    // the quotient where `inside(a)`, with no branch
-    __device__ __forceinline__ double fast(double a) const {
-        const double q0 = a * y;
-        const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
-        return __fma_rn(__fma_rn(-b, q1, a), y, q1);
-    }
-    __device__ __forceinline__ bool inside(double a) const {   // 2^-895 <= |a| < 2^770
-        return ok_b && ((unsigned)__double2hiint(a) & 0x7fffffffu) - 0x08000000u <= 0x68000000u;
-    }
-    __device__ __forceinline__ double of(double a) const { return inside(a) ? fast(a) : a / b; }
-};
-
 __device__ __forceinline__ int bitrev(int i, int logn) { return (int)(__brev((unsigned)i) >> (32 - logn)); }
 
 // Shared-memory slot of element i of a transform line: a spare slot after every
@@ -242,8 +217,7 @@ __device__ __forceinline__ void fft_turn(Cplx<T>* a, int LS, int n, int logn, do
     constexpr int M = 1 << H;
     const int gpl = n >> H, l = threadIdx.x % CW, q = threadIdx.x / CW;
     const bool mine = q < gpl;
-    const SharedDivisor by_Ly(Ly);
-    const double two_pi = 2.0 * M_PI;
+    const double two_pi = 2.0 * M_PI, inv_Ly = 1.0 / Ly;
     Cplx<T> y[M];
     if (mine) {
         Cplx<T> x[M];
@@ -253,7 +227,7 @@ __device__ __forceinline__ void fft_turn(Cplx<T>* a, int LS, int n, int logn, do
 #pragma unroll
         for (int m = 0; m < M; m++) {
             const int j = q + m * gpl, nj = (j <= n / 2) ? j : j - n;
-            const double ky = by_Ly.of(two_pi * (double)nj);
+            const double ky = quotient(two_pi * (double)nj, Ly, inv_Ly);
             const double k2 = kx * kx + ky * ky;
             const T f = (k2 == 0.0) ? T(0) : (T)(-fourpiG / k2);
             // the inverse's first pass takes element rev(m) n/2^H + q as its m-th
@@ -770,7 +744,8 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
         });
     };
     cl.sync();
-    const SharedDivisor denom(a.denom), cells((double)N);
+    const double inv_denom = 1.0 / a.denom, cells = (double)N, inv_cells = 1.0 / cells;
+    const bool denom_ok = divisor_inside(a.denom);
     const double omega = a.omega, idx2 = a.idx2, idy2 = a.idy2, tol = a.tol;
     double m = 0.0;   // mean removal pending on every cell not yet rewritten in this sweep
     double res = 0.0;
@@ -788,7 +763,7 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
     };
     // whether the quotient a / denom needs the division (an extreme a; a zero does not)
     auto extreme = [&](double q) {
-        return !denom.inside(q) && (__double2loint(q) | (__double2hiint(q) & 0x7fffffff)) != 0;
+        return !(denom_ok && quotient_inside(q));
     };
     // max |lap(phi - m) - rhs| over the thread's cells
     auto residual = [&]() {
@@ -843,10 +818,10 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
             }
             if (rare) {
 #pragma unroll
-                for (int v = 0; v < V; v++) q[v] = q[v] / denom.b;
+                for (int v = 0; v < V; v++) q[v] = q[v] / a.denom;
             } else {
 #pragma unroll
-                for (int v = 0; v < V; v++) q[v] = denom.fast(q[v]);
+                for (int v = 0; v < V; v++) q[v] = quotient_fast(q[v], a.denom, inv_denom);
             }
 #pragma unroll
             for (int v = 0; v < V; v++) {
@@ -877,10 +852,10 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
             }
             if (rare) {
 #pragma unroll
-                for (int v = 0; v < V; v++) q[v] = q[v] / denom.b;
+                for (int v = 0; v < V; v++) q[v] = q[v] / a.denom;
             } else {
 #pragma unroll
-                for (int v = 0; v < V; v++) q[v] = denom.fast(q[v]);
+                for (int v = 0; v < V; v++) q[v] = quotient_fast(q[v], a.denom, inv_denom);
             }
 #pragma unroll
             for (int v = 0; v < V; v++) {
@@ -921,7 +896,7 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
                 double t = 0.0;
 #pragma unroll 8
                 for (int q = 0; q < nb; q++) t += pt[q];
-                s_val = cells.of(t);
+                s_val = quotient(t, cells, inv_cells);
             }
         }
         if (edge) wait(BLACK, ph);
