@@ -42,6 +42,29 @@ int default_march_rows(int nx, int ny) {
     if (rows > 128) rows = 128;
     return (int)rows;
 }
+// The FP32 stage of a grid: rows per warp of the register march, or 0 where the
+// tiles are faster.  The march has few, long chains (a row takes a lone warp
+// 1.2 us), so a grid needs warps: four strips to a CTA, four CTAs to an SM, and
+// a row costs 1.2, 1.35, 1.75 or 2.2 us with one to four CTAs on it; a segment
+// pays three rows to start.  The tiles take 6.6 us a wave of one to an SM, 9.5
+// of two, and 8.2 us for every further 296.  The march has to be 8% ahead in
+// this count, for its errors; the line lies near 500^2.  Steps without gravity,
+// tiles and best march: 256^2 33.8 and 35.6 us, 384^2 42.9 either way, 512^2
+// 58.7 and 52.9, 900 x 700 103 and 96, 1003 x 777 122 and 99, 2048^2 588 and
+// 457, 4096^2 2252 and 1576.
+int lane_rows(int nx, int ny) {
+    auto div_up = [](long a, long b) { return (a + b - 1) / b; };
+    const long tiles = div_up(nx, 30) * div_up(ny, 15);
+    double best = 0.92 * (tiles <= 148 ? 6.6 : (tiles <= 296 ? 9.5 : 8.2 * (double)tiles / 296.0));
+    int rows = 0;
+    static constexpr double row_us[5] = {0.0, 1.2, 1.35, 1.75, 2.2};
+    for (int seg = 2; seg <= 64; seg += 2) {
+        const long ctas = div_up(div_up(nx, 28), 4) * div_up(ny, seg);
+        const double us = (seg + 3) * ((double)(ctas / 592) * row_us[4] + row_us[div_up(ctas % 592, 148)]);
+        if (us < best) { best = us; rows = seg; }
+    }
+    return rows;
+}
 int ilog2(int n) { int l = 0; while ((1 << l) < n) ++l; return l; }
 
 // --------------------------------------------------------------------------
@@ -76,8 +99,11 @@ template <class T> struct Mhd2d : Mhd2dBase {
     bool comp = false;
     void* lblock = nullptr;
     Fields<T> lbuf[3];
-    // stage kernel: CC_STAGE_TILE (the default; FP64's only form) or CC_STAGE_MARCH (FP32)
-    int stage_kind = CC_STAGE_TILE;
+    // stage kernel: STAGE_AUTO (the register march in segments of lane_seg rows, or the tiles) until
+    // cc_mhd2d_set_stage_kernel asks for CC_STAGE_TILE or CC_STAGE_MARCH
+    static constexpr int STAGE_AUTO = -1;
+    int stage_kind = STAGE_AUTO;
+    int lane_seg = 0;     // 0: tiles (FP64, a compensated state, a small grid)
     int march_rows = 0;   // 0: from the grid (init)
     int cur = 0;
     T* phi = nullptr;
@@ -148,6 +174,7 @@ template <class T> struct Mhd2d : Mhd2dBase {
         if (p.compensated && sizeof(T) != 4)
             return fail(h, CC_ERR_UNSUPPORTED, "the compensated update is an option of the FP32 path");
         comp = p.compensated != 0;
+        lane_seg = (sizeof(T) == 4 && !comp) ? lane_rows(nx, ny) : 0;
         CC_CUDA(cudaMalloc(&block, sizeof(T) * plane * 24));
         CC_CUDA(cudaMemsetAsync(block, 0, sizeof(T) * plane * 24, st()));
         for (int b = 0; b < 3; b++) {
@@ -400,7 +427,9 @@ template <class T> struct Mhd2d : Mhd2dBase {
             CC_CUDA(cudaEventCreate(&e1));
             CC_CUDA(cudaEventRecord(e0, st()));
         }
-        if (stage_kind == CC_STAGE_MARCH)
+        if (stage_kind == STAGE_AUTO && lane_seg > 0)
+            CC_CUDA(M2Launch<T>::stage_lane(c, buf[bi], buf[bo], defer, gmode, ga, gb, dt_dev, active(), lane_seg, st()));
+        else if (stage_kind == CC_STAGE_MARCH)
             CC_CUDA(M2Launch<T>::stage_march(c, buf[bi], buf[bo], comp ? &lbuf[bi] : nullptr,
                                              comp ? &lbuf[bo] : nullptr, defer, gmode, ga, gb, dt_dev, active(),
                                              march_rows, st()));

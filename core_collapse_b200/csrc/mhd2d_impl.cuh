@@ -1,5 +1,6 @@
 // Definitions of M2Launch<T>; included once per precision TU.
 #pragma once
+#include "mhd2d_lane.cuh"
 #include "mhd2d_launch.h"
 
 namespace ccb {
@@ -162,6 +163,31 @@ cudaError_t M2Launch<T>::stage_comp(const M2Const<T>& c, const Fields<T>& in, co
         CC_STAGE_CASE(true, GRAV_ARRAYS)
         CC_STAGE_CASE(true, GRAV_PHI)
 #undef CC_STAGE_CASE
+        return cudaErrorInvalidValue;
+    }
+}
+
+template <class T>
+cudaError_t M2Launch<T>::stage_lane(const M2Const<T>& c, const Fields<T>& in, const Fields<T>& out, bool defer, int gmode,
+                                    const T* ga, const T* gb, const double* dt, const int* active, int seg, cudaStream_t s) {
+    if constexpr (sizeof(T) != 4) {
+        return cudaErrorNotSupported;
+    } else {
+        if (seg < 1) return cudaErrorInvalidValue;
+        const int strips = (c.nx + LANE_W - 1) / LANE_W, per = LANE_NT / 32;
+        const dim3 grid((strips + per - 1) / per, (c.ny + seg - 1) / seg);
+#define CC_LANE_CASE(D, G)                                                                             \
+        if (defer == D && gmode == G) {                                                                \
+            m2_lane_kernel<D, G><<<grid, LANE_NT, 0, s>>>(c, in, out, ga, gb, dt, active, seg);         \
+            return cudaGetLastError();                                                                 \
+        }
+        CC_LANE_CASE(false, GRAV_NONE)
+        CC_LANE_CASE(false, GRAV_ARRAYS)
+        CC_LANE_CASE(false, GRAV_PHI)
+        CC_LANE_CASE(true, GRAV_NONE)
+        CC_LANE_CASE(true, GRAV_ARRAYS)
+        CC_LANE_CASE(true, GRAV_PHI)
+#undef CC_LANE_CASE
         return cudaErrorInvalidValue;
     }
 }

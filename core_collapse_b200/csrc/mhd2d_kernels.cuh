@@ -94,14 +94,8 @@ template <class T> constexpr size_t m2_stage_smem() { return StageGeom<T>::smem;
 // |J|^2 and the 5-point Laplacian of Bz of cell (i,j) of the stored state s,
 // whose own Bz is bzC (M2:640-668)
 template <class T>
-__device__ __forceinline__ void joule_terms(const M2Const<T>& c, const Fields<T>& s, int i, int j, T bzC, T& J2,
-                                            T& lap) {
-    const int P = c.pitch;
-    const int iE = c.ax.cell(i + 1), iW = c.ax.cell(i - 1);
-    const int jN = c.ay.cell(j + 1), jS = c.ay.cell(j - 1);
-    const T bzE = s.Bz[(size_t)j * P + iE], bzW = s.Bz[(size_t)j * P + iW];
-    const T bzN = s.Bz[(size_t)jN * P + i], bzS = s.Bz[(size_t)jS * P + i];
-    const T dby = s.by[(size_t)j * P + iE] - s.by[(size_t)j * P + i], dbx = s.bx[(size_t)jN * P + i] - s.bx[(size_t)j * P + i];
+__device__ __forceinline__ void joule_from(const M2Const<T>& c, T bzE, T bzW, T bzN, T bzS, T bzC, T dby, T dbx, T& J2,
+                                           T& lap) {
     J2 = divided<T>([&](auto& d) {
         const T dBzdy = d.quot_by(bzN - bzS, c.two_dy, T(0.5) * c.inv_dy);
         const T dBzdx = d.quot_by(bzE - bzW, c.two_dx, T(0.5) * c.inv_dx);
@@ -111,6 +105,24 @@ __device__ __forceinline__ void joule_terms(const M2Const<T>& c, const Fields<T>
         return Jx * Jx + Jy * Jy + Jz * Jz;
     });
     lap = (bzE - T(2) * bzC + bzW) * c.idx2 + (bzN - T(2) * bzC + bzS) * c.idy2;
+}
+template <class T>
+__device__ __forceinline__ void joule_terms(const M2Const<T>& c, const Fields<T>& s, int i, int j, T bzC, T& J2,
+                                            T& lap) {
+    const int P = c.pitch;
+    const int iE = c.ax.cell(i + 1), iW = c.ax.cell(i - 1);
+    const int jN = c.ay.cell(j + 1), jS = c.ay.cell(j - 1);
+    joule_from(c, s.Bz[(size_t)j * P + iE], s.Bz[(size_t)j * P + iW], s.Bz[(size_t)jN * P + i], s.Bz[(size_t)jS * P + i], bzC,
+               s.by[(size_t)j * P + iE] - s.by[(size_t)j * P + i], s.bx[(size_t)jN * P + i] - s.bx[(size_t)j * P + i], J2, lap);
+}
+
+// eta J_z of an edge from the differences of By across it in x and of Bx in y (M2:565-575)
+template <class T> __device__ __forceinline__ T resistive_emf(const M2Const<T>& c, T dby, T dbx) {
+    return divided<T>([&](auto& d) {
+        const T dBydx = d.quot_by(dby, c.dx, c.inv_dx);
+        const T dBxdy = d.quot_by(dbx, c.dy, c.inv_dy);
+        return c.eta * (dBydx - dBxdy);
+    });
 }
 
 template <class T>
@@ -410,11 +422,7 @@ __device__ __forceinline__ void m2_stage_tile(const M2Const<T>& c, const Fields<
             const int cj = c.ay.cell(je), cjm = c.ay.cell(je - 1);
             const T dby = in.by[(size_t)je * P + ci] - in.by[(size_t)je * P + cim];
             const T dbx = in.bx[(size_t)cj * P + ie] - in.bx[(size_t)cjm * P + ie];
-            res = divided<T>([&](auto& d) {
-                const T dBydx = d.quot_by(dby, c.dx, c.inv_dx);
-                const T dBxdy = d.quot_by(dbx, c.dy, c.inv_dy);
-                return c.eta * (dBydx - dBxdy);
-            });
+            res = resistive_emf(c, dby, dbx);
         }
         ez[k] = ideal + res;
     }

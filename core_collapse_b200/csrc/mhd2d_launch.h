@@ -32,6 +32,9 @@ template <class T> struct M2Launch {
                                     double* rho_part, cudaStream_t s);
     // FP32 column-march stage (mhd2d_march.cuh): segments of seg_rows rows;
     // lin / lout non-null: compensated state
+    // FP32: the stage as a march of warps in registers (mhd2d_lane.cuh), seg rows to a warp
+    static cudaError_t stage_lane(const M2Const<T>& c, const Fields<T>& in, const Fields<T>& out, bool defer, int gmode,
+                                  const T* ga, const T* gb, const double* dt, const int* active, int seg, cudaStream_t s);
     static cudaError_t stage_march(const M2Const<T>& c, const Fields<T>& in, const Fields<T>& out,
                                    const Fields<T>* lin, const Fields<T>* lout, bool defer, int gmode, const T* ga,
                                    const T* gb, const double* dt, const int* active, int seg_rows, cudaStream_t s);

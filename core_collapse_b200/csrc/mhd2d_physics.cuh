@@ -403,6 +403,23 @@ __device__ __forceinline__ Prim<float> lane_y(const Prim2& S) {
     return Prim<float>{S.r.y, S.u.y, S.v.y, S.w.y, S.P.y, S.bx.y, S.by.y, S.bz.y};
 }
 
+// Energy flux of ideal_flux with the fused multiply-adds spelled out, those that
+// the compiler forms in the tile kernel's y faces (there the sums start with the
+// second of their first two products); vB: its v . B.
+__device__ __forceinline__ float energy_flux_y(const M2Const<float>& c, const Prim<float>& W, float& vB) {
+    const float B2 = fmaf(W.bz, W.bz, fmaf(W.by, W.by, __fmul_rn(W.bx, W.bx)));
+    const float k = fmaf(W.w, W.w, fmaf(W.u, W.u, __fmul_rn(W.v, W.v)));
+    vB = fmaf(W.w, W.bz, fmaf(W.u, W.bx, __fmul_rn(W.v, W.by)));
+    const float E = fmaf(0.5f, B2, fmaf(W.P, 1.0f / c.gm1, __fmul_rn(__fmul_rn(0.5f, W.r), k)));
+    const float pt = fmaf(0.5f, B2, W.P);
+    return fmaf(E + pt, W.u, -__fmul_rn(W.bx, vB));
+}
+
+// YSUM: the energy flux's sums as energy_flux_y has them.  These sums of two
+// products can be fused in two ways, and which one the compiler takes depends on
+// the order in which the kernel around forms u and v: the register march
+// (mhd2d_lane.cuh) asks for the tile kernel's.
+template <bool YSUM = false>
 __device__ __forceinline__ Flux<float> hlld_x2(const M2Const<float>& c, Prim2 S, const float Bn) {
     const float2 bn = pbc(Bn);
     S.bx = bn;
@@ -421,8 +438,14 @@ __device__ __forceinline__ Flux<float> hlld_x2(const M2Const<float>& c, Prim2 S,
     const float2 um = psub(S.u, cf), up = padd(S.u, cf);
     const float SL = fminf(um.x, um.y);
     const float SR = fmaxf(up.x, up.y);
-    if (0.0f <= SL) return ideal_flux(c, lane_x(S));
-    if (0.0f >= SR) return ideal_flux(c, lane_y(S));
+    auto flux_of = [&](const Prim<float>& W) {
+        Flux<float> F = ideal_flux(c, W);
+        float vB;
+        if (YSUM) F.f4 = energy_flux_y(c, W, vB);
+        return F;
+    };
+    if (0.0f <= SL) return flux_of(lane_x(S));
+    if (0.0f >= SR) return flux_of(lane_y(S));
 
     // energies and total pressures (M2:357, 482, 495)
     const float2 ksum = pfma(S.w, S.w, pfma(S.v, S.v, pmul(S.u, S.u)));
@@ -432,7 +455,7 @@ __device__ __forceinline__ Flux<float> hlld_x2(const M2Const<float>& c, Prim2 S,
 
     if (fabsf(Bn) < 1e-12f) {  // HLL (M2:449-467)
         const Prim<float> L = lane_x(S), R = lane_y(S);
-        const Flux<float> FL = ideal_flux(c, L), FR = ideal_flux(c, R);
+        const Flux<float> FL = flux_of(L), FR = flux_of(R);
         const float inv = 1.0f / (SR - SL);
         const float s2 = SL * SR;
         Flux<float> F;
@@ -495,10 +518,14 @@ __device__ __forceinline__ Flux<float> hlld_x2(const M2Const<float>& c, Prim2 S,
         Bys = (sq.x * Bys2.y + sq.y * Bys2.x + sq.x * sq.y * (vs2.y - vs2.x) * sgn) * id2;
         Bzs = (sq.x * Bzs2.y + sq.y * Bzs2.x + sq.x * sq.y * (ws2.y - ws2.x) * sgn) * id2;
     }
-    const float vBs = SM * Bn + vs * Bys + ws * Bzs;
-    const float vBw = W.u * W.bx + W.v * W.by + W.w * W.bz;
-    const float Es = ((Sw - W.u) * EW - (ptW * W.u - Bn * vBw) + (pts * SM - Bn * vBs)) / (Sw - SM);
     Flux<float> F = ideal_flux(c, W);
+    float vBs = SM * Bn + vs * Bys + ws * Bzs;
+    float vBw = W.u * W.bx + W.v * W.by + W.w * W.bz;
+    if (YSUM) {
+        vBs = fmaf(ws, Bzs, fmaf(SM, Bn, __fmul_rn(vs, Bys)));
+        F.f4 = energy_flux_y(c, W, vBw);
+    }
+    const float Es = ((Sw - W.u) * EW - (ptW * W.u - Bn * vBw) + (pts * SM - Bn * vBs)) / (Sw - SM);
     F.f0 = F.f0 + Sw * (rs - W.r);
     F.f1 = F.f1 + Sw * (rs * SM - W.r * W.u);
     F.f2 = F.f2 + Sw * (rs * vs - W.r * W.v);

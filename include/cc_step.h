@@ -255,12 +255,14 @@ int cc_mhd2d_rk2_step(cc_handle* h, const double* gx, const double* gy, double d
 int cc_mhd2d_advance(cc_handle* h, int nsteps, double* t);
 
 /* Choice of the stage kernel (no counterpart in the reference, whose
- * advance_stage M2:690-834 is one function): CC_STAGE_TILE, the default, one
- * CTA per tile of cells with a recomputed halo (the only form for FP64), or
- * CC_STAGE_MARCH, FP32 only, a CTA per column strip that
- * marches up a segment of seg_rows rows carrying the rows below it (0: a
- * length chosen from the grid so the segments fill the GPU).  Both evaluate
- * the same expressions; a tuning and testing switch. */
+ * advance_stage M2:690-834 is one function): CC_STAGE_TILE, one CTA per tile of
+ * cells with a recomputed halo (the only form for FP64), or CC_STAGE_MARCH,
+ * FP32 only, a CTA per column strip that marches up a segment of seg_rows rows
+ * carrying the rows below it (0: a length chosen from the grid so the segments
+ * fill the GPU).  A handle that is not asked for one of them runs the tiles, or
+ * on an uncompensated FP32 grid large enough to fill the GPU with them, warps
+ * that march in registers.  All evaluate the same expressions; a tuning and
+ * testing switch. */
 #define CC_STAGE_TILE 0
 #define CC_STAGE_MARCH 1
 int cc_mhd2d_set_stage_kernel(cc_handle* h, int kind, int seg_rows);
