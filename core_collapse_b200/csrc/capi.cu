@@ -43,24 +43,18 @@ int default_march_rows(int nx, int ny) {
     return (int)rows;
 }
 // The FP32 stage of a grid: rows per warp of the register march, or 0 where the
-// tiles are faster.  The march has few, long chains (a row takes a lone warp
-// 1.2 us), so a grid needs warps: four strips to a CTA, four CTAs to an SM, and
-// a row costs 1.2, 1.35, 1.75 or 2.2 us with one to four CTAs on it; a segment
-// pays three rows to start.  The tiles take 6.6 us a wave of one to an SM, 9.5
-// of two, and 8.2 us for every further 296.  The march has to be 8% ahead in
-// this count, for its errors; the line lies near 500^2.  Steps without gravity,
+// tiles are faster by the counts of mhd2d_launch.h.  The march has to be 8%
+// ahead, for their errors; the line lies near 500^2.  Steps without gravity,
 // tiles and best march: 256^2 33.8 and 35.6 us, 384^2 42.9 either way, 512^2
 // 58.7 and 52.9, 900 x 700 103 and 96, 1003 x 777 122 and 99, 2048^2 588 and
 // 457, 4096^2 2252 and 1576.
 int lane_rows(int nx, int ny) {
     auto div_up = [](long a, long b) { return (a + b - 1) / b; };
-    const long tiles = div_up(nx, 30) * div_up(ny, 15);
-    double best = 0.92 * (tiles <= 148 ? 6.6 : (tiles <= 296 ? 9.5 : 8.2 * (double)tiles / 296.0));
+    double best = 0.92 * stage_tiles_us(div_up(nx, 30) * div_up(ny, 15));
     int rows = 0;
-    static constexpr double row_us[5] = {0.0, 1.2, 1.35, 1.75, 2.2};
     for (int seg = 2; seg <= 64; seg += 2) {
-        const long ctas = div_up(div_up(nx, 28), 4) * div_up(ny, seg);
-        const double us = (seg + 3) * ((double)(ctas / 592) * row_us[4] + row_us[div_up(ctas % 592, 148)]);
+        if (div_up(ny, seg) > 65535) continue;   // grid.y
+        const double us = stage_lane_us(div_up(div_up(nx, 28), 4) * div_up(ny, seg), seg);
         if (us < best) { best = us; rows = seg; }
     }
     return rows;

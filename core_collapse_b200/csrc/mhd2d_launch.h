@@ -14,6 +14,18 @@ namespace ccb {
 constexpr int RED_NT = 512;      // threads of the reduction kernels (two blocks per SM at <= 64 registers)
 constexpr int RED_BLOCKS = 296;  // 2 x 148 SMs; fixed so reduction order is fixed
 
+// What an FP32 stage takes (us, without gravity), to choose between the tiles
+// and the register march.  The march has few, long chains (a row takes a lone
+// warp 1.2 us): a row costs 1.2, 1.35, 1.75 or 2.2 us with one to four CTAs of
+// four strips to an SM, and a segment pays three rows to start.  The tiles take
+// 8.2 us for every 296, one wave of two to an SM; grids of one wave are theirs
+// without a count (a step at 64^2: 23.5 us, 24.9 with the march of two rows).
+inline double stage_tiles_us(long tiles) { return tiles <= 296 ? 0.0 : 8.2 * (double)tiles / 296.0; }
+inline double stage_lane_us(long ctas, int rows) {
+    static constexpr double row_us[5] = {0.0, 1.2, 1.35, 1.75, 2.2};
+    return (rows + 3) * ((double)(ctas / 592) * row_us[4] + row_us[(ctas % 592 + 147) / 148]);
+}
+
 template <class T> struct M2Launch {
     // raise the dynamic shared-memory limits of the kernels (once per device, before any launch or capture)
     static cudaError_t prepare(int nx, int ny);
