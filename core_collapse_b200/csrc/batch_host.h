@@ -123,6 +123,10 @@ template <class T> struct Batch : BatchBase {
     std::vector<int2*> swork;        // per stage shape
     std::vector<int> nswork;
     std::vector<int> sgrid;          // CTAs per candidate
+    // FP32: the register march, which runs unless it is the slower one by its
+    // count (nlwork 0) or by autotune, or a tile candidate was set
+    int2* lwork = nullptr; int nlwork = 0;
+    bool lane = false;
     int2* rwork = nullptr; int nrwork = 0;
     int2* gwork = nullptr; int ngwork = 0; int gtile = 64;
     int2* tcwork = nullptr; int ntcwork = 0;   // FP32 instances with 16-byte rows: tcgen05 transforms
@@ -173,6 +177,34 @@ template <class T> struct Batch : BatchBase {
         if (int r = dalloc(ptr, v.size())) return r;
         if (!v.empty()) CC_CUDA(cudaMemcpyAsync(*ptr, v.data(), sizeof(U) * v.size(), cudaMemcpyHostToDevice, st()));
         return CC_OK;
+    }
+
+    // Work-list of the register march: the segment length for which the
+    // instances' (strip, segment) pairs, four to a CTA, take the least time by the
+    // counts of mhd2d_launch.h (with the 8% that a single grid asks of the march),
+    // each instance's segments then of equal length; empty where the tiles are
+    // faster, as for a batch of one wave of tiles.
+    std::vector<int2> lane_work() const {
+        std::vector<int2> w;
+        if (sizeof(T) != 4) return w;
+        auto div_up = [](long a, long b) { return (a + b - 1) / b; };
+        auto ctas = [&](int i, int rows) { return div_up(div_up(p[i].Nx, LANE_W) * div_up(p[i].Ny, rows), LANE_NT / 32); };
+        long tiles = 0;
+        for (int i = 0; i < n; i++) tiles += div_up(p[i].Nx, 30) * div_up(p[i].Ny, 15);
+        double best = 0.92 * stage_tiles_us(tiles);
+        int rows = 0;
+        for (int k = 2; k <= 126; k += 2) {
+            long sum = 0, most = 0;
+            for (int i = 0; i < n; i++) { sum += ctas(i, k); most = std::max(most, ctas(i, k)); }
+            const double us = stage_lane_us(sum, k);
+            if (us < best && most < (1L << 24)) { best = us; rows = k; }
+        }
+        if (rows == 0) return w;
+        for (int i = 0; i < n; i++) {
+            const int mine = (int)div_up(p[i].Ny, div_up(p[i].Ny, rows));
+            for (long k = 0; k < ctas(i, mine); k++) w.push_back(make_int2(i, mine << 24 | (int)k));
+        }
+        return w;
     }
 
     int init() override {
@@ -337,6 +369,10 @@ template <class T> struct Batch : BatchBase {
             sgrid[k] = std::max(1, std::min(nswork[k], per_sm * nsm));
             sgrid[NS + k] = std::max(1, nswork[k]);
         }
+        const std::vector<int2> lw = lane_work();
+        nlwork = (int)lw.size();
+        lane = nlwork > 0;
+        if (int r = upload_vec(&lwork, lw)) return r;
         if (int r = upload_vec(&dinst, hinst)) return r;
         if (int r = upload_vec(&dred, hred)) return r;
         if (int r = dalloc(&spd_part, nrwork)) return r;
@@ -448,8 +484,11 @@ template <class T> struct Batch : BatchBase {
             CC_CUDA(cudaEventRecord(e0, st()));
         }
         const int k = shape % BatchLaunch<T>::n_shapes();
-        CC_CUDA(BatchLaunch<T>::stage(k, sgrid[shape], dinst, swork[k], nswork[k], src, dst_, defer, any_grav, dt,
-                                      active, st()));
+        if (lane)
+            CC_CUDA(BatchLaunch<T>::stage_lane(dinst, lwork, nlwork, src, dst_, defer, any_grav, dt, active, st()));
+        else
+            CC_CUDA(BatchLaunch<T>::stage(k, sgrid[shape], dinst, swork[k], nswork[k], src, dst_, defer, any_grav, dt,
+                                          active, st()));
         count(1);
         if (h->profiling) {
             CC_CUDA(cudaEventRecord(e1, st()));
@@ -600,10 +639,25 @@ template <class T> struct Batch : BatchBase {
             const double per = (double)ms / reps;
             if (per < best_ms) { best_ms = per; best = c; }
         }
+        bool march = false;
+        if (nlwork > 0) {
+            float ms = 0.f;
+            CC_CUDA(BatchLaunch<T>::stage_lane(dinst, lwork, nlwork, cur, b, false, any_grav, dt, active, st()));
+            CC_CUDA(cudaEventRecord(e0, st()));
+            for (int r = 0; r < reps; r++)
+                CC_CUDA(BatchLaunch<T>::stage_lane(dinst, lwork, nlwork, cur, b, false, any_grav, dt, active, st()));
+            CC_CUDA(cudaEventRecord(e1, st()));
+            CC_CUDA(cudaEventSynchronize(e1));
+            CC_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+            count(reps + 1);
+            march = (double)ms / reps < best_ms;
+            if (march) best_ms = (double)ms / reps;
+        }
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        if (best != shape) invalidate_graph();
+        if (best != shape || march != lane) invalidate_graph();
         shape = best;
+        lane = march;
         if (out_shape) *out_shape = best;
         if (out_ms) *out_ms = best_ms;
         return CC_OK;
@@ -611,8 +665,9 @@ template <class T> struct Batch : BatchBase {
 
     int set_shape(int k) override {
         if (k < 0 || k >= 2 * BatchLaunch<T>::n_shapes()) return fail(h, CC_ERR_ARG, "no such stage candidate");
-        if (k != shape) invalidate_graph();
+        if (k != shape || lane) invalidate_graph();
         shape = k;
+        lane = false;
         return CC_OK;
     }
 

@@ -155,6 +155,20 @@ cudaError_t BatchLaunch<T>::stage(int k, int grid, const BatchInst<T>* inst, con
 }
 
 template <class T>
+cudaError_t BatchLaunch<T>::stage_lane(const BatchInst<T>* inst, const int2* work, int nwork, int src, int dst,
+                                       bool defer, bool grav, const double* dt, const int* active, cudaStream_t s) {
+    if constexpr (sizeof(T) != 4) {
+        return cudaErrorNotSupported;
+    } else {
+        if (defer && grav) m2b_lane_kernel<true, GRAV_PHI><<<nwork, LANE_NT, 0, s>>>(inst, work, src, dst, dt, active);
+        else if (defer) m2b_lane_kernel<true, GRAV_NONE><<<nwork, LANE_NT, 0, s>>>(inst, work, src, dst, dt, active);
+        else if (grav) m2b_lane_kernel<false, GRAV_PHI><<<nwork, LANE_NT, 0, s>>>(inst, work, src, dst, dt, active);
+        else m2b_lane_kernel<false, GRAV_NONE><<<nwork, LANE_NT, 0, s>>>(inst, work, src, dst, dt, active);
+        return cudaGetLastError();
+    }
+}
+
+template <class T>
 cudaError_t BatchLaunch<T>::average(const BatchInst<T>* inst, const int2* rwork, int nrwork, int a, int d, int b,
                                     const double* dt, const int* active, double* spd_part, double* rho_part,
                                     cudaStream_t s) {

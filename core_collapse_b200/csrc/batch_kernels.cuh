@@ -19,6 +19,7 @@
 //                 other instances in the batch.
 #pragma once
 #include "mhd2d_kernels.cuh"
+#include "mhd2d_lane.cuh"
 
 namespace ccb {
 
@@ -98,6 +99,34 @@ m2b_stage_kernel(const BatchInst<T>* __restrict__ inst, const int2* __restrict__
                                                         nullptr, (T)dt[it.x], tx * TX, ty * TY, sm, s_inst.rec);
         __syncthreads();                            // shared tile buffers reused by the next tile
     }
+}
+
+// ---------------------------------------------------------------------------
+// The FP32 stage as the register march of mhd2d_lane.cuh: a work item is an
+// instance, a segment length and four (strip, segment) pairs of that instance,
+// one to a warp, so that instances of one or two strips fill their CTAs too.
+// Same bits as the tiles.  128 square instances of 64 to 256 cells a side (164 on
+// average) with gravity, first / second stage: tiles 317 / 343 us -> 185 / 222.
+// The instance's constants and planes are copied out of shared memory first:
+// read there they are loaded again in every row (192 / 235 us).
+// ---------------------------------------------------------------------------
+template <bool DEFER, int GMODE>
+__global__ void __launch_bounds__(LANE_NT, 4)
+m2b_lane_kernel(const BatchInst<float>* __restrict__ inst, const int2* __restrict__ work, int src, int dst,
+                const double* __restrict__ dt, const int* __restrict__ active) {
+    __shared__ __align__(16) BatchInst<float> s_inst;
+    __shared__ LaneKeep keep;
+    const int2 it = work[blockIdx.x];
+    if (active[it.x] == 0) return;                  // uniform over the CTA
+    load_inst(&s_inst, inst + it.x);
+    const M2Const<float> c = s_inst.c;
+    const Fields<float> in = s_inst.buf[src], out = s_inst.buf[dst];
+    const int rows = it.y >> 24, t = (it.y & 0xffffff) * (LANE_NT / 32) + (threadIdx.x >> 5);
+    const int strips = (c.nx + LANE_W - 1) / LANE_W;
+    const int j0 = t / strips * rows;
+    if (j0 >= c.ny) return;                         // whole warps
+    m2_lane_segment<DEFER, GMODE, ESUM_BATCH>(keep, c, in, out, s_inst.phi, nullptr, (float)dt[it.x], t % strips,
+                                  j0, min(j0 + rows, c.ny));
 }
 
 // ---------------------------------------------------------------------------

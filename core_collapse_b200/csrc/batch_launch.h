@@ -23,6 +23,9 @@ template <class T> struct BatchLaunch {
     static cudaError_t resident(int k, int* per_sm);
     static cudaError_t stage(int k, int grid, const BatchInst<T>* inst, const int2* work, int nwork, int src, int dst,
                              bool defer, bool grav, const double* dt, const int* active, cudaStream_t s);
+    // FP32: the stage as a register march over its own work-list (m2b_lane_kernel)
+    static cudaError_t stage_lane(const BatchInst<T>* inst, const int2* work, int nwork, int src, int dst, bool defer,
+                                  bool grav, const double* dt, const int* active, cudaStream_t s);
     // stage with the record of the pre-floor update (inst->rec), tile candidate 0, one CTA per tile
     static cudaError_t stage_rec(const BatchInst<T>* inst, const int2* work, int nwork, int src, int dst, bool defer,
                                  bool grav, const double* dt, const int* active, cudaStream_t s);

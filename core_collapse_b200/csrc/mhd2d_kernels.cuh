@@ -93,7 +93,8 @@ template <class T> constexpr size_t m2_stage_smem() { return StageGeom<T>::smem;
 // E, Bz, rho are updated.  Bx, By are the cell-centred stage-output B.
 // |J|^2 and the 5-point Laplacian of Bz of cell (i,j) of the stored state s,
 // whose own Bz is bzC (M2:640-668)
-template <class T>
+// ES: the sums' products fused as in the tile kernels (FP32)
+template <class T, ESum ES = ESUM_FREE>
 __device__ __forceinline__ void joule_from(const M2Const<T>& c, T bzE, T bzW, T bzN, T bzS, T bzC, T dby, T dbx, T& J2,
                                            T& lap) {
     J2 = divided<T>([&](auto& d) {
@@ -102,9 +103,12 @@ __device__ __forceinline__ void joule_from(const M2Const<T>& c, T bzE, T bzW, T 
         const T dBydx = d.quot_by(dby, c.dx, c.inv_dx);
         const T dBxdy = d.quot_by(dbx, c.dy, c.inv_dy);
         const T Jx = dBzdy, Jy = -dBzdx, Jz = dBydx - dBxdy;
-        return Jx * Jx + Jy * Jy + Jz * Jz;
+        if constexpr (ES == ESUM_GRID) return dot_spelled(Jy, Jy, Jx, Jx, Jz, Jz);
+        else if constexpr (ES == ESUM_BATCH) return dot_spelled(Jx, Jx, Jy, Jy, Jz, Jz);
+        else return Jx * Jx + Jy * Jy + Jz * Jz;
     });
-    lap = (bzE - T(2) * bzC + bzW) * c.idx2 + (bzN - T(2) * bzC + bzS) * c.idy2;
+    if constexpr (ES != ESUM_FREE) lap = fmaf(bzE - T(2) * bzC + bzW, c.idx2, __fmul_rn(bzN - T(2) * bzC + bzS, c.idy2));
+    else lap = (bzE - T(2) * bzC + bzW) * c.idx2 + (bzN - T(2) * bzC + bzS) * c.idy2;
 }
 template <class T>
 __device__ __forceinline__ void joule_terms(const M2Const<T>& c, const Fields<T>& s, int i, int j, T bzC, T& J2,

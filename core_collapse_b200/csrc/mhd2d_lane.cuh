@@ -13,7 +13,7 @@
 // segment starts with 2 rows of x faces and 4 of primitives.
 //
 // Same expressions as the tile kernel and the same contractions, so the same
-// bits (the energy flux of the y faces needs them spelled out: hlld_x2<true>).
+// bits (the energy flux needs them spelled out: ESum).
 // That is kept on purpose: some FP32 runs amplify a last bit to 1e-3 of a weak
 // field within a hundred steps, so a cheaper HLLD with shared reciprocals (598 /
 // 715 us below) would have changed their results.
@@ -21,7 +21,7 @@
 // Bound: issue (65% of the slots at 16 warps an SM; 128 registers allow no more,
 // and 20 warps at 96 registers spilled: 722 us) and the latency of a row's two
 // HLLD chains.  4096^2 with gravity, first / second stage of a step: tiles 1103
-// / 1156 us -> 655 / 767.  On the way: the potential carried instead of read at
+// / 1156 us -> 661 / 778.  On the way: the potential carried instead of read at
 // the update (717 -> 611 with the cheaper HLLD: a load there is waited for), the
 // state before the update kept in shared memory instead of read again and the
 // Joule sub-step from shuffles (864 -> 715, second stage).  1003 x 777: 51 / 54
@@ -62,7 +62,7 @@ struct LaneKeep {
     float4 f[3][LANE_NT];
 };
 
-template <bool DEFER, int GMODE>
+template <bool DEFER, int GMODE, ESum ES>
 __device__ __forceinline__ void m2_lane_segment(LaneKeep& keep, const M2Const<float>& c, const Fields<float>& in, const Fields<float>& out,
                                                 const float* __restrict__ ga, const float* __restrict__ gb, const float dt,
                                                 const int strip, const int j0, const int j1) {
@@ -119,7 +119,7 @@ __device__ __forceinline__ void m2_lane_segment(LaneKeep& keep, const M2Const<fl
             if (r == j0 - 2 || c.ay.cell(r - 1) != cjS) zS = in.Bz[(size_t)cjS * P + ci];
             const float zC = Bz;
             float J2, lap;
-            joule_from(c, zE, zW, raw.zN, zS, zC, yE - raw.y0, raw.bN - raw.b0, J2, lap);
+            joule_from<float, ES>(c, zE, zW, raw.zN, zS, zC, yE - raw.y0, raw.bN - raw.b0, J2, lap);
             E = E + dt * c.eta * J2;
             Bz = zC + dt * c.eta * lap;
             floors(c, rho, mx, my, mz, E, Bx, By, Bz);
@@ -153,7 +153,7 @@ __device__ __forceinline__ void m2_lane_segment(LaneKeep& keep, const M2Const<fl
                 S.P = pk(fmaxf(xl.P, c.floor_P), fmaxf(xr.P, c.floor_P));
                 S.u = pk(xl.u, xr.u); S.v = pk(xl.v, xr.v); S.w = pk(xl.w, xr.w);
                 S.bx = pbc(bn); S.by = pk(xl.bt, xr.bt); S.bz = pk(xl.bz, xr.bz);
-                const Flux<float> F = hlld_x2(c, S, bn);
+                const Flux<float> F = hlld_x2<ES>(c, S, bn);
                 Fx[0] = F.f0; Fx[1] = F.f1; Fx[2] = F.f2; Fx[3] = F.f3; Fx[4] = F.f4; Fx[5] = F.f5; Fx[6] = F.f6;
             }
             // ---- y face r - 1, between rows r - 2 and r - 1; edges and faces of that row ----
@@ -165,7 +165,7 @@ __device__ __forceinline__ void m2_lane_segment(LaneKeep& keep, const M2Const<fl
                 S.P = pk(fmaxf(plus.P, c.floor_P), fmaxf(lo.P, c.floor_P));
                 S.u = pk(plus.v, lo.v); S.v = pk(plus.u, lo.u); S.w = pk(plus.w, lo.w);
                 S.bx = pbc(bnY); S.by = pk(plus.bt, lo.bt); S.bz = pk(plus.bz, lo.bz);
-                const Flux<float> F = hlld_x2<true>(c, S, bnY);
+                const Flux<float> F = hlld_x2<ES>(c, S, bnY);
                 Gy[0] = F.f0; Gy[1] = F.f2; Gy[2] = F.f1; Gy[3] = F.f3; Gy[4] = F.f4; Gy[5] = F.f5; Gy[6] = F.f6;
                 // edge EMF at the lower left corner of the row's cells (M2:782-804)
                 const float exm = -F5, ex0 = -Fx[5], ey0 = Gy[5], eym = lane_up(ey0);
@@ -247,7 +247,7 @@ m2_lane_kernel(const M2Const<float> c, const Fields<float> in, const Fields<floa
     const int j0 = blockIdx.y * seg, j1 = j0 + seg < c.ny ? j0 + seg : c.ny;
     if (strip * LANE_W >= c.nx) return;   // whole warps
     __shared__ LaneKeep keep;
-    m2_lane_segment<DEFER, GMODE>(keep, c, in, out, ga, gb, (float)*dtp, strip, j0, j1);
+    m2_lane_segment<DEFER, GMODE, ESUM_GRID>(keep, c, in, out, ga, gb, (float)*dtp, strip, j0, j1);
 }
 
 }  // namespace ccb

@@ -403,23 +403,32 @@ __device__ __forceinline__ Prim<float> lane_y(const Prim2& S) {
     return Prim<float>{S.r.y, S.u.y, S.v.y, S.w.y, S.P.y, S.bx.y, S.by.y, S.bz.y};
 }
 
-// Energy flux of ideal_flux with the fused multiply-adds spelled out, those that
-// the compiler forms in the tile kernel's y faces (there the sums start with the
-// second of their first two products); vB: its v . B.
-__device__ __forceinline__ float energy_flux_y(const M2Const<float>& c, const Prim<float>& W, float& vB) {
+// Some sums of two products, in the energy flux and the Joule heating, can be
+// fused in two ways, and which one the compiler takes depends on the order in which
+// the kernel around forms the operands.  The register march (mhd2d_lane.cuh) has them
+// spelled out as they are in the tile kernel of a single grid or in that of a batch,
+// which differ in the internal and kinetic energy and in J^2, so that a grid has the
+// same bits in either form.
+enum ESum { ESUM_FREE, ESUM_GRID, ESUM_BATCH };
+
+// a x + b y + c z, spelled out as above
+__device__ __forceinline__ float dot_spelled(float a, float x, float b, float y, float c, float z) {
+    return fmaf(c, z, fmaf(a, x, __fmul_rn(b, y)));
+}
+// energy flux of ideal_flux in that form; vB: its v . B
+template <ESum ES>
+__device__ __forceinline__ float energy_flux(const M2Const<float>& c, const Prim<float>& W, float& vB) {
     const float B2 = fmaf(W.bz, W.bz, fmaf(W.by, W.by, __fmul_rn(W.bx, W.bx)));
-    const float k = fmaf(W.w, W.w, fmaf(W.u, W.u, __fmul_rn(W.v, W.v)));
-    vB = fmaf(W.w, W.bz, fmaf(W.u, W.bx, __fmul_rn(W.v, W.by)));
-    const float E = fmaf(0.5f, B2, fmaf(W.P, 1.0f / c.gm1, __fmul_rn(__fmul_rn(0.5f, W.r), k)));
+    const float k = dot_spelled(W.u, W.u, W.v, W.v, W.w, W.w);
+    vB = dot_spelled(W.u, W.bx, W.v, W.by, W.w, W.bz);
+    const float ig = 1.0f / c.gm1, hr = __fmul_rn(0.5f, W.r);
+    const float ek = ES == ESUM_GRID ? fmaf(W.P, ig, __fmul_rn(hr, k)) : fmaf(hr, k, __fmul_rn(W.P, ig));
+    const float E = fmaf(0.5f, B2, ek);
     const float pt = fmaf(0.5f, B2, W.P);
     return fmaf(E + pt, W.u, -__fmul_rn(W.bx, vB));
 }
 
-// YSUM: the energy flux's sums as energy_flux_y has them.  These sums of two
-// products can be fused in two ways, and which one the compiler takes depends on
-// the order in which the kernel around forms u and v: the register march
-// (mhd2d_lane.cuh) asks for the tile kernel's.
-template <bool YSUM = false>
+template <ESum ES = ESUM_FREE>
 __device__ __forceinline__ Flux<float> hlld_x2(const M2Const<float>& c, Prim2 S, const float Bn) {
     const float2 bn = pbc(Bn);
     S.bx = bn;
@@ -440,8 +449,10 @@ __device__ __forceinline__ Flux<float> hlld_x2(const M2Const<float>& c, Prim2 S,
     const float SR = fmaxf(up.x, up.y);
     auto flux_of = [&](const Prim<float>& W) {
         Flux<float> F = ideal_flux(c, W);
-        float vB;
-        if (YSUM) F.f4 = energy_flux_y(c, W, vB);
+        if constexpr (ES != ESUM_FREE) {
+            float vB;
+            F.f4 = energy_flux<ES>(c, W, vB);
+        }
         return F;
     };
     if (0.0f <= SL) return flux_of(lane_x(S));
@@ -519,13 +530,18 @@ __device__ __forceinline__ Flux<float> hlld_x2(const M2Const<float>& c, Prim2 S,
         Bzs = (sq.x * Bzs2.y + sq.y * Bzs2.x + sq.x * sq.y * (ws2.y - ws2.x) * sgn) * id2;
     }
     Flux<float> F = ideal_flux(c, W);
-    float vBs = SM * Bn + vs * Bys + ws * Bzs;
-    float vBw = W.u * W.bx + W.v * W.by + W.w * W.bz;
-    if (YSUM) {
-        vBs = fmaf(ws, Bzs, fmaf(SM, Bn, __fmul_rn(vs, Bys)));
-        F.f4 = energy_flux_y(c, W, vBw);
+    float Es;
+    if constexpr (ES != ESUM_FREE) {
+        float vBw;
+        F.f4 = energy_flux<ES>(c, W, vBw);
+        const float vBs = dot_spelled(SM, Bn, vs, Bys, ws, Bzs);
+        const float wW = fmaf(ptW, W.u, -__fmul_rn(Bn, vBw)), wS = fmaf(pts, SM, -__fmul_rn(Bn, vBs));
+        Es = (fmaf(Sw - W.u, EW, -wW) + wS) / (Sw - SM);
+    } else {
+        const float vBs = SM * Bn + vs * Bys + ws * Bzs;
+        const float vBw = W.u * W.bx + W.v * W.by + W.w * W.bz;
+        Es = ((Sw - W.u) * EW - (ptW * W.u - Bn * vBw) + (pts * SM - Bn * vBs)) / (Sw - SM);
     }
-    const float Es = ((Sw - W.u) * EW - (ptW * W.u - Bn * vBw) + (pts * SM - Bn * vBs)) / (Sw - SM);
     F.f0 = F.f0 + Sw * (rs - W.r);
     F.f1 = F.f1 + Sw * (rs * SM - W.r * W.u);
     F.f2 = F.f2 + Sw * (rs * vs - W.r * W.v);

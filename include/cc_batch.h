@@ -75,7 +75,9 @@ int cc_batch_times(cc_handle* h, double* t);
  * keep the fastest; shape / ms (may be NULL) receive the choice and its mean
  * stage time.  Candidate c uses tile shape c % S of the S compiled shapes,
  * launched persistent (c < S: one CTA per resident slot walking a contiguous
- * run of the tile work-list) or flat (c >= S: one CTA per tile). */
+ * run of the tile work-list) or flat (c >= S: one CTA per tile).  An FP32 batch
+ * of more than a wave of tiles runs its stages as warps that march in registers,
+ * with the same bits, until a candidate is set or is found here to be faster. */
 int cc_batch_autotune(cc_handle* h, int reps, int* shape, double* ms);
 /* Use candidate `shape` (0 <= shape < n_shapes). */
 int cc_batch_set_shape(cc_handle* h, int shape);
