@@ -55,8 +55,9 @@ template <class T>
 cudaError_t M3Launch<T>::emf_ct(const M3Const<T>& c, const Fields3<T>& in, const Fields3<T>& out, const FaceData<T>& X,
                                 const FaceData<T>& Y, const FaceData<T>& Z, const double* dt, const int* active,
                                 cudaStream_t st) {
-    const dim3 g((c.nx + 1 + 30) / 31, (c.ny + 1 + 6) / 7, (c.nz + 1 + M3_EDGE_KCH - 1) / M3_EDGE_KCH);
-    m3_emf_ct_kernel<T><<<g, 256, 0, st>>>(c, in, out, X, Y, Z, dt, active);
+    const int kch = m3_edge_kch(c.nx, c.ny, c.nz);
+    const dim3 g((c.nx + 1 + 30) / 31, (c.ny + 1 + 6) / 7, (c.nz + 1 + kch - 1) / kch);
+    m3_emf_ct_kernel<T><<<g, 256, 0, st>>>(c, in, out, X, Y, Z, dt, active, kch);
     return cudaGetLastError();
 }
 

@@ -90,14 +90,17 @@ __device__ __forceinline__ T joule3_cc(const M3Const<T>& c, const Bcc3<T>& b, in
     auto at = [&](const T* f, int a, int bb, int d) { return f[c.idx(a, bb, d)]; };
     const int ip = c.ax.cell(i + 1), im = c.ax.cell(i - 1), jp = c.ay.cell(j + 1), jm = c.ay.cell(j - 1);
     const int kp = c.az.cell(k + 1), km = c.az.cell(k - 1);
-    const T dBzdy = (at(b.z, i, jp, k) - at(b.z, i, jm, k)) / c.two_dy;
-    const T dBydz = (at(b.y, i, j, kp) - at(b.y, i, j, km)) / c.two_dz;
-    const T dBxdz = (at(b.x, i, j, kp) - at(b.x, i, j, km)) / c.two_dz;
-    const T dBzdx = (at(b.z, ip, j, k) - at(b.z, im, j, k)) / c.two_dx;
-    const T dBydx = (at(b.y, ip, j, k) - at(b.y, im, j, k)) / c.two_dx;
-    const T dBxdy = (at(b.x, i, jp, k) - at(b.x, i, jm, k)) / c.two_dy;
-    const T Jx = dBzdy - dBydz, Jy = dBxdz - dBzdx, Jz = dBydx - dBxdy;
-    const T J2 = Jx * Jx + Jy * Jy + Jz * Jz;
+    const T by_z = at(b.z, i, jp, k) - at(b.z, i, jm, k), bz_y = at(b.y, i, j, kp) - at(b.y, i, j, km);
+    const T bz_x = at(b.x, i, j, kp) - at(b.x, i, j, km), bx_z = at(b.z, ip, j, k) - at(b.z, im, j, k);
+    const T bx_y = at(b.y, ip, j, k) - at(b.y, im, j, k), by_x = at(b.x, i, jp, k) - at(b.x, i, jm, k);
+    const T hx = T(0.5) * c.inv_dx, hy = T(0.5) * c.inv_dy, hz = T(0.5) * c.inv_dz;
+    const T J2 = divided<T>([&](auto& d) {
+        const T dBzdy = d.quot_by(by_z, c.two_dy, hy), dBydz = d.quot_by(bz_y, c.two_dz, hz);
+        const T dBxdz = d.quot_by(bz_x, c.two_dz, hz), dBzdx = d.quot_by(bx_z, c.two_dx, hx);
+        const T dBydx = d.quot_by(bx_y, c.two_dx, hx), dBxdy = d.quot_by(by_x, c.two_dy, hy);
+        const T Jx = dBzdy - dBydz, Jy = dBxdz - dBzdx, Jz = dBydx - dBxdy;
+        return Jx * Jx + Jy * Jy + Jz * Jz;
+    });
     return dt * c.eta * J2;
 }
 
@@ -364,6 +367,14 @@ template <class T> struct EdgeColumn {
         }
     }
 
+    // eta (d1 / h1 - d2 / h2)
+    __device__ __forceinline__ T curl(T d1, T h1, T i1, T d2, T h2, T i2) const {
+        return divided<T>([&](auto& d) {
+            const T a = d.quot_by(d1, h1, i1), b = d.quot_by(d2, h2, i2);
+            return c.eta * (a - b);
+        });
+    }
+
     // the three EMFs of plane k (0 where the edge does not exist), then advance
     __device__ __forceinline__ void step(int k, T& ex, T& ey, T& ez) {
         const int ck = c.az.cell(k), fk = c.az.face(k), fk1 = c.az.face(k + 1);
@@ -378,9 +389,8 @@ template <class T> struct EdgeColumn {
             const T ideal = T(0.25) * (exy_p + exy_k + at(Z.f[5], ci, cjm, fk) + at(Z.f[5], ci, cj, fk));
             T res = T(0.0);
             if (res_on) {
-                const T dBzdy = (T(0.5) * (bz0 + bz1) - T(0.5) * (bz0s + bz1s)) / c.dy;
-                const T dBydz = (by_k - by_p) / c.dz;
-                res = c.eta * (dBzdy - dBydz);
+                const T dbz = T(0.5) * (bz0 + bz1) - T(0.5) * (bz0s + bz1s), dby = by_k - by_p;
+                res = curl(dbz, c.dy, c.inv_dy, dby, c.dz, c.inv_dz);
             }
             ex = ideal + res;
         }
@@ -388,9 +398,8 @@ template <class T> struct EdgeColumn {
             const T ideal = T(0.25) * (eyx_p + eyx_k + at(Z.f[6], cim, cj, fk) + at(Z.f[6], ci, cj, fk));
             T res = T(0.0);
             if (res_on) {
-                const T dBxdz = (bx_k - bx_p) / c.dz;
-                const T dBzdx = (T(0.5) * (bz0 + bz1) - T(0.5) * (bz0w + bz1w)) / c.dx;
-                res = c.eta * (dBxdz - dBzdx);
+                const T dbx = bx_k - bx_p, dbz = T(0.5) * (bz0 + bz1) - T(0.5) * (bz0w + bz1w);
+                res = curl(dbx, c.dz, c.inv_dz, dbz, c.dx, c.inv_dx);
             }
             ey = ideal + res;
         }
@@ -399,9 +408,8 @@ template <class T> struct EdgeColumn {
                                        at(Y.f[5], ci, fj, ck));
             T res = T(0.0);
             if (res_on) {
-                const T dBydx = (by_k - byc(cim, ck)) / c.dx;
-                const T dBxdy = (bx_k - bxc(cjm, ck)) / c.dy;
-                res = c.eta * (dBydx - dBxdy);
+                const T dby = by_k - byc(cim, ck), dbx = bx_k - bxc(cjm, ck);
+                res = curl(dby, c.dx, c.inv_dx, dbx, c.dy, c.inv_dy);
             }
             ez = ideal + res;
         }
@@ -412,7 +420,7 @@ template <class T> struct EdgeColumn {
 
 // Edge EMFs and the CT update of the three face arrays in one pass (M3:879-939
 // then M3:942-1015).  A CTA of 32 x 8 threads owns the faces of 31 x 7 (i, j)
-// columns over a chunk of M3_EDGE_KCH planes; each thread marches one edge
+// columns over a chunk of kch planes (a multiple of M3_EMF_KB); each thread marches one edge
 // column (EdgeColumn: the 32nd column and 8th row are the neighbours the
 // owned faces read).  The march goes in bricks of M3_EMF_KB planes: a thread
 // forms the EMFs of the brick's M3_EMF_KB + 1 edge planes (no barrier in
@@ -426,12 +434,22 @@ template <class T> struct EdgeColumn {
 // 6.65 ms, FP64 16.32 -> 16.16 ms, three edge planes less memory (the edge
 // march is latency-bound, and the saved traffic is small beside it); with a
 // barrier pair per plane instead of per brick it was 1% slower.
-constexpr int M3_EDGE_KCH = 32;
 constexpr int M3_EMF_KB = 4;
+// kch: 32 planes, halved while that leaves fewer than 592 CTAs (four to an SM; a
+// chunk pays one more edge plane): 90 x 70 x 52 in FP64 is 66 CTAs of 32 planes,
+// 135 us, and 462 of 4 planes, 36 (with the quotients of the resistive EMF free of
+// branches; 256^3 in FP32 keeps 32 planes: 576 -> 544).
+inline int m3_edge_kch(int nx, int ny, int nz) {
+    const long columns = (long)((nx + 31) / 31) * ((ny + 7) / 7);
+    int kch = 32;
+    while (kch > M3_EMF_KB && columns * ((nz + kch) / kch) < 592) kch /= 2;
+    return kch;
+}
 template <class T>
 __global__ void __launch_bounds__(256) m3_emf_ct_kernel(const M3Const<T> c, const Fields3<T> in, const Fields3<T> out,
                                                         const FaceData<T> X, const FaceData<T> Y, const FaceData<T> Z,
-                                                        const double* __restrict__ dtp, const int* __restrict__ active) {
+                                                        const double* __restrict__ dtp, const int* __restrict__ active,
+                                                        const int kch) {
     if (active && *active == 0) return;
     constexpr int KB = M3_EMF_KB;
     __shared__ T sx[KB + 1][8][32], sy[KB + 1][8][32], sz[KB + 1][8][32];
@@ -439,8 +457,8 @@ __global__ void __launch_bounds__(256) m3_emf_ct_kernel(const M3Const<T> c, cons
     const int i = blockIdx.x * 31 + tx, j = blockIdx.y * 7 + ty;
     const bool live = i <= c.nx && j <= c.ny;
     const bool owner = live && tx < 31 && ty < 7;
-    const int k0 = blockIdx.z * M3_EDGE_KCH;
-    const int k1 = min(c.nz + 1, k0 + M3_EDGE_KCH);   // Bz planes k0 .. k1-1 of this chunk
+    const int k0 = blockIdx.z * kch;
+    const int k1 = min(c.nz + 1, k0 + kch);   // Bz planes k0 .. k1-1 of this chunk
     const int kend = min(k1, c.nz);                    // edge planes k0 .. kend
     const T dt = (T)(*dtp);
     const T dtdx = dt / c.dx, dtdy = dt / c.dy, dtdz = dt / c.dz;
