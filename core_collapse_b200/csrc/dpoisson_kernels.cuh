@@ -120,134 +120,137 @@ dp_gemm_kernel(const BatchInst<T>* __restrict__ inst, const int2* __restrict__ g
 // y solves: one thread per x wavenumber k >= 1 (a warp covers 32 adjacent
 // wavenumbers, so every row access is one coalesced 256-byte line), the
 // singular k = 0 on a CTA of its own.  Each sweep is a chain of fma's whose
-// loads do not depend on the chain: rows are fetched YB at a time into
-// registers one block ahead of the block being computed, which overlaps the
-// L2 latency with the chain.  The arithmetic and its order are those of the
-// CPU restatement (bitwise).
-constexpr int YB = 16;
+// loads do not depend on the chain, and a grid has few of these warps, so a sweep
+// takes its chain only if its rows are under way long before: column and factors
+// by cp.async in a ring of shared memory, YB rows to a group, YD - 1 groups ahead
+// of the group being computed (registers that hold rows under way cannot be passed
+// on from group to group without waiting for them: one group ahead is all they
+// give).  The arithmetic and its order are those of the CPU restatement (bitwise).
+// One clamped 512^2 in FP64: 93 -> 41 us; 128 FP32 instances of 64 to 256 cells a
+// side: 52 -> 26.
+constexpr int YB = 8, YD = 8;
+template <class T> using YRing = T[2][YD][YB][DPC];
 
-// forward sweep: d_0 = u_0 inv_0, d_j = (u_j - a d_{j-1}) inv_j, u_j <- d_j; returns d_{n-1}
-// (the prefetch of the block after the last one reads clamped, in-range rows)
-template <class S_>
-__device__ __forceinline__ S_ ysweep_fwd(S_* __restrict__ u, const S_* __restrict__ inv, size_t S, int n, S_ a) {
-    S_ d = u[0] * inv[0];
-    u[0] = d;
-    int j = 1;
-    const int nb = (n - 1) / YB;
-    S_ cu[YB], ci[YB];
-#pragma unroll
-    for (int t = 0; t < YB; t++) {
-        const int r = min(j + t, n - 1);
-        cu[t] = u[r * S]; ci[t] = inv[r * S];
-    }
-    for (int b = 0; b < nb; b++, j += YB) {
-        S_ nu[YB], ni[YB];
-#pragma unroll
-        for (int t = 0; t < YB; t++) {
-            const int r = min(j + YB + t, n - 1);
-            nu[t] = u[r * S]; ni[t] = inv[r * S];
-        }
-#pragma unroll
-        for (int t = 0; t < YB; t++) {
-            d = fma(-a, d, cu[t]) * ci[t];
-            u[(j + t) * S] = d;
-        }
-#pragma unroll
-        for (int t = 0; t < YB; t++) { cu[t] = nu[t]; ci[t] = ni[t]; }
-    }
-    for (; j < n; j++) {
-        d = fma(-a, d, u[j * S]) * inv[j * S];
-        u[j * S] = d;
-    }
-    return d;
+template <class S_> __device__ __forceinline__ void y_fetch(S_* smem, const S_* g) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g),
+                 "n"(sizeof(S_)) : "memory");
 }
 
-// backward sweep: x_{n-1} = d_{n-1}, x_j = d_j - cp_j x_{j+1}, u_j <- x_j; returns x_0
-template <class S_>
-__device__ __forceinline__ S_ ysweep_bwd(S_* __restrict__ u, const S_* __restrict__ cp, size_t S, int n, S_ x) {
-    int j = n - 2;
-    const int nb = (n - 1) / YB;
-    S_ cu[YB], cc[YB];
-#pragma unroll
-    for (int t = 0; t < YB; t++) {
-        const int r = max(j - t, 0);
-        cu[t] = u[r * S]; cc[t] = cp[r * S];
-    }
-    for (int b = 0; b < nb; b++, j -= YB) {
-        S_ nu[YB], nc[YB];
+// u_i <- f(u_i, w_i) for the rows i < n in turn, row i at u + i St, w + i St
+template <class S_, class F>
+__device__ __forceinline__ void ysweep(S_* u, const S_* w, YRing<S_>& ring, ptrdiff_t St, int n, F f) {
+    const int lane = threadIdx.x;
+    __threadfence_block();   // the sweep before wrote the rows that the copies read
+    auto fetch = [&](int g) {
+        const S_* pu = u + (ptrdiff_t)g * YB * St;
+        const S_* pw = w + (ptrdiff_t)g * YB * St;
 #pragma unroll
         for (int t = 0; t < YB; t++) {
-            const int r = max(j - YB - t, 0);
-            nu[t] = u[r * S]; nc[t] = cp[r * S];
+            if (g * YB + t < n) {
+                y_fetch(&ring[0][g % YD][t][lane], pu);
+                y_fetch(&ring[1][g % YD][t][lane], pw);
+            }
+            pu += St; pw += St;
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int g = 0; g < YD - 1; g++) fetch(g);
+    for (int g = 0; g * YB < n; g++) {
+        fetch(g + YD - 1);   // into the slots of group g - 1
+        asm volatile("cp.async.wait_group %0;" ::"n"(YD - 1) : "memory");   // group g is there
+        S_ uv[YB], wv[YB];
+#pragma unroll
+        for (int t = 0; t < YB; t++) { uv[t] = ring[0][g % YD][t][lane]; wv[t] = ring[1][g % YD][t][lane]; }
+        S_* p = u + (ptrdiff_t)g * YB * St;
 #pragma unroll
         for (int t = 0; t < YB; t++) {
-            x = fma(-cc[t], x, cu[t]);
-            u[(j - t) * S] = x;
+            if (g * YB + t < n) *p = f(uv[t], wv[t]);
+            p += St;
         }
+    }
+}
+
+// The singular k = 0 by a warp: flux G_j = a (u_{j+1} - u_j) = G_{j-1} + r_j, then
+// the mean removed.  A lane loads and stores a row of 32; every lane runs the
+// chain, on rows handed round by shuffles.
+template <class T> __device__ __forceinline__ void ysolve_singular(T* u, size_t S, int n, bool py, T dy2) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x;
+    auto row = [&](int j) { return j < n ? u[j * S] : T(0); };
+    T g0 = T(0);
+    if (py) {
+        T Sr = T(0), SS = T(0), v = row(lane);
+        for (int j = 0; j < n; j += 32) {
+            const T nv = row(j + 32 + lane);
 #pragma unroll
-        for (int t = 0; t < YB; t++) { cu[t] = nu[t]; cc[t] = nc[t]; }
+            for (int t = 0; t < 32; t++) {
+                const T r = __shfl_sync(ALL, v, t);
+                if (j + t < n) { Sr = Sr + r; SS = SS + Sr; }
+            }
+            v = nv;
+        }
+        g0 = -(SS / (T)n);
     }
-    for (; j >= 0; j--) {
-        x = fma(-cp[j * S], x, u[j * S]);
-        u[j * S] = x;
+    T G = g0, prev = T(0), m = T(0), v = row(lane);
+    for (int j = 0; j < n; j += 32) {
+        const T nv = row(j + 32 + lane);
+        T mine = T(0);
+#pragma unroll
+        for (int t = 0; t < 32; t++) {
+            const T r = __shfl_sync(ALL, v, t);
+            if (lane == t) mine = prev;
+            if (j + t < n) {
+                m = m + prev;
+                G = G + r;
+                prev = fma(dy2, G, prev);
+            }
+        }
+        if (j + lane < n) u[(j + lane) * S] = mine;
+        v = nv;
     }
-    return x;
+    m = m / (T)n;
+    for (int j = lane; j < n; j += 32 * 8) {
+        T q[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) q[t] = row(j + 32 * t);
+#pragma unroll
+        for (int t = 0; t < 8; t++)
+            if (j + 32 * t < n) u[(j + 32 * t) * S] = q[t] - m;
+    }
 }
 
 template <class T>
 __global__ void __launch_bounds__(DPC)
 dp_ysolve_kernel(const BatchInst<T>* __restrict__ inst, const int2* __restrict__ ywork, int nywork,
                  const int* __restrict__ active) {
+    __shared__ YRing<T> ring;
     for (int w = blockIdx.x; w < nywork; w += gridDim.x) {
         const int2 it = ywork[w];
         if (active[it.x] == 0) continue;
         const BatchInst<T>& I = inst[it.x];
         const int nx = I.c.nx, n = I.c.ny;
-        const size_t S = (size_t)nx;
+        const ptrdiff_t S = nx;
         const bool py = I.c.ay.periodic != 0;
         const T a = (T)I.ay;
         if (it.y < 0) {
-            // singular k = 0: flux G_j = a (u_{j+1} - u_j) = G_{j-1} + r_j, then mean removal
-            if (threadIdx.x != 0) continue;
-            T* __restrict__ u = I.ah;
-            T g0 = T(0);
-            if (py) {
-                T Sr = T(0), SS = T(0);
-#pragma unroll 16
-                for (int j = 0; j < n; j++) { Sr = Sr + u[j * S]; SS = SS + Sr; }
-                g0 = -(SS / (T)n);
-            }
-            const T dy2 = (T)I.dy2;
-            T G = g0, prev = T(0);
-            T r = u[0];
-            u[0] = T(0);
-#pragma unroll 16
-            for (int j = 0; j + 1 < n; j++) {
-                G = G + r;
-                r = u[(j + 1) * S];
-                prev = fma(dy2, G, prev);
-                u[(j + 1) * S] = prev;
-            }
-            T m = T(0);
-#pragma unroll 16
-            for (int j = 0; j < n; j++) m = m + u[j * S];
-            m = m / (T)n;
-#pragma unroll 16
-            for (int j = 0; j < n; j++) u[j * S] = u[j * S] - m;
+            ysolve_singular(I.ah, (size_t)nx, n, py, (T)I.dy2);
             continue;
         }
         const int col = 1 + it.y * DPC + threadIdx.x;
         if (col >= nx) continue;
-        T* __restrict__ u = I.ah + col;
-        const T d = ysweep_fwd<T>(u, I.yinv + col, S, n, a);
-        const T x = ysweep_bwd<T>(u, I.ycp + col, S, n, d);
+        T* u = I.ah + col;
+        // forward: d_0 = u_0 inv_0, d_j = (u_j - a d_{j-1}) inv_j, u_j <- d_j
+        T d = u[0] * I.yinv[col];
+        u[0] = d;
+        ysweep(u + S, I.yinv + col + S, ring, S, n - 1, [&](T uj, T inv) { return d = fma(-a, d, uj) * inv; });
+        // backward: x_{n-1} = d_{n-1}, x_j = d_j - cp_j x_{j+1}, u_j <- x_j
+        T x = d;
+        ysweep(u + (n - 2) * S, I.ycp + col + (n - 2) * S, ring, -S, n - 1, [&](T uj, T cp) { return x = fma(-cp, x, uj); });
         if (!py) continue;
-        const T* __restrict__ z = I.yz + col;
         const T gam = -fma(T(-2), a, I.lamx[col]);
         const T fac = fma(a / gam, d, x) * I.yfden[col];   // d = x_{n-1}, x = x_0
-#pragma unroll 8
-        for (int j = 0; j < n; j++) u[j * S] = fma(-fac, z[j * S], u[j * S]);
+        ysweep(u, I.yz + col, ring, S, n, [&](T uj, T z) { return fma(-fac, z, uj); });
     }
 }
 
