@@ -145,6 +145,9 @@ template <class T> struct Batch : BatchBase {
     double* diag_part = nullptr;
     double* staging = nullptr;
     size_t staging_elems = 0;
+    static constexpr size_t DOWN_HALF = (size_t)4 << 20;   // bytes; pinned, two of them to a handle
+    char* down = nullptr;
+    cudaEvent_t down_done[2] = {nullptr, nullptr};
     bool any_grav = false;
     int shape = 0;
     int cur = 0;
@@ -162,6 +165,9 @@ template <class T> struct Batch : BatchBase {
 
     ~Batch() override {
         if (graph3) cudaGraphExecDestroy(graph3);
+        for (cudaEvent_t e : down_done)
+            if (e) cudaEventDestroy(e);
+        if (down) cudaFreeHost(down);
         for (void* q : allocs) cudaFree(q);
     }
 
@@ -383,7 +389,11 @@ template <class T> struct Batch : BatchBase {
         if (int r = dalloc(&active, n)) return r;
         if (int r = dalloc(&steps, n)) return r;
         if (int r = dalloc(&diag_part, (size_t)RED_BLOCKS * 7)) return r;
-        if (int r = dalloc(&staging, staging_elems)) return r;
+        if (int r = dalloc(&staging, std::max(staging_elems, DOWN_HALF / sizeof(double)))) return r;
+        void* pin = nullptr;
+        if (cudaHostAlloc(&pin, 2 * DOWN_HALF, cudaHostAllocDefault) == cudaSuccess) down = static_cast<char*>(pin);
+        else cudaGetLastError();   // downloads then copy field by field
+        for (cudaEvent_t& e : down_done) CC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         CC_CUDA(cudaMemsetAsync(dt, 0, sizeof(double) * n, st()));
         CC_CUDA(cudaMemsetAsync(tclk, 0, sizeof(double) * n, st()));
         CC_CUDA(cudaMemsetAsync(rho_mean, 0, sizeof(double) * n, st()));
@@ -435,11 +445,57 @@ template <class T> struct Batch : BatchBase {
         layout(i, w, hh);
         const Fields<T>& B = hinst[i].buf[cur];
         const T* src[8] = {B.rho, B.mx, B.my, B.mz, B.E, B.Bz, B.bx, B.by};
+        // Pageable destinations go through two pinned halves of DOWN_HALF bytes: as
+        // many fields as fit are packed and copied by one transfer, and copied out of
+        // one half while the next transfer fills the other (a larger field takes
+        // pieces of its own).  Copied by itself into pageable memory, a field makes the
+        // driver stage it and wait: 128 instances of 64 to 256 cells a side took
+        // 135 ms into new arrays, and 96 this way (most of it their first touch).
+        struct Part { int field; size_t src, off, bytes; };   // of a field, from byte src, to byte off of the half
+        std::vector<std::vector<Part>> pieces;
+        size_t used = DOWN_HALF;                               // of the last piece
         for (int k = 0; k < 8; k++) {
             if (!f[k]) continue;
-            CC_CUDA(M2Launch<T>::pack_out(src[k], staging, w[k], hh[k], pitch[i], st()));
-            CC_CUDA(cudaMemcpyAsync(f[k], staging, sizeof(double) * (size_t)w[k] * hh[k], cudaMemcpyDeviceToHost, st()));
-            h->perf.kernel_launches += 1;
+            const size_t all = sizeof(double) * (size_t)w[k] * hh[k];
+            cudaPointerAttributes at{};
+            const bool pageable = cudaPointerGetAttributes(&at, f[k]) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
+            cudaGetLastError();
+            if (!pageable || !down) {
+                CC_CUDA(M2Launch<T>::pack_out(src[k], staging, w[k], hh[k], pitch[i], st()));
+                CC_CUDA(cudaMemcpyAsync(f[k], staging, all, cudaMemcpyDeviceToHost, st()));
+                h->perf.kernel_launches += 1;
+            } else if (all > DOWN_HALF) {
+                for (size_t b = 0; b < all; b += DOWN_HALF) pieces.push_back({Part{k, b, 0, std::min(all - b, DOWN_HALF)}});
+                used = DOWN_HALF;
+            } else {
+                if (used + all > DOWN_HALF) { pieces.emplace_back(); used = 0; }
+                pieces.back().push_back(Part{k, 0, used, all});
+                used += all;
+            }
+        }
+        auto issue = [&](size_t q) -> int {
+            size_t bytes = 0;
+            for (const Part& x : pieces[q]) {
+                if (x.src == 0) {
+                    CC_CUDA(M2Launch<T>::pack_out(src[x.field], staging + x.off / sizeof(double), w[x.field], hh[x.field],
+                                                  pitch[i], st()));
+                    h->perf.kernel_launches += 1;
+                }
+                bytes += x.bytes;
+            }
+            const double* from = staging + pieces[q].front().src / sizeof(double);
+            CC_CUDA(cudaMemcpyAsync(down + (q & 1) * DOWN_HALF, from, bytes, cudaMemcpyDeviceToHost, st()));
+            CC_CUDA(cudaEventRecord(down_done[q & 1], st()));
+            return CC_OK;
+        };
+        if (!pieces.empty())
+            if (int r = issue(0)) return r;
+        for (size_t q = 0; q < pieces.size(); q++) {
+            if (q + 1 < pieces.size())
+                if (int r = issue(q + 1)) return r;
+            CC_CUDA(cudaEventSynchronize(down_done[q & 1]));
+            for (const Part& x : pieces[q])
+                std::memcpy(reinterpret_cast<char*>(f[x.field]) + x.src, down + (q & 1) * DOWN_HALF + x.off, x.bytes);
         }
         CC_CUDA(cudaStreamSynchronize(st()));
         return CC_OK;
