@@ -21,27 +21,30 @@ template <class T> __host__ __device__ constexpr T tiny_pos() { return sizeof(T)
 __host__ __device__ __forceinline__ int wrap_idx(int i, int n) { int r = i % n; return (r < 0) ? r + n : r; }
 __host__ __device__ __forceinline__ int clamp_idx(int i, int lo, int hi) { return i < lo ? lo : (i > hi ? hi : i); }
 
-// Correctly rounded FP64 quotients without a branch.  A division is 13
-// operations on the FP64 pipe and ends in a branch to its slow path, so that
-// one waits for the other: a chain of 120 cycles each (107 cycles of a warp's
-// issue instead of 27 when the numerator is a zero, which the velocity and
-// field components that a planar flow does not have are).  The forms below
+// Correctly rounded FP64 quotients without a branch.  A division waits for the
+// one before it: measured, a chain of 120 cycles each, and 107 cycles of a
+// warp's issue instead of 27 when the numerator is a zero, which the velocity and
+// field components that a planar flow does not have are.  The forms below
 // overlap, and quotients of one denominator share its reciprocal.
-//   y = RN(1/b): the hardware's approximation, one third-order Newton step (an
-//   error below 2^-59 before its rounding, so y is within one ulp), and one step
-//   that rounds it correctly, unless b's significand is all ones.
+//   y = RN(1/b): two Newton-Raphson steps y <- y + y (1 - b y), each of which
+//   squares the relative error, from a starting value within 2^-14: 2^-28, then
+//   2^-56 before the rounding of y, so y is within one ulp; then one more step,
+//   which rounds it correctly unless b's significand is all ones.
 //   a / b from y: q0 = a y is within two ulps, q1 = q0 + (a - b q0) y is a
 //   faithful quotient, and from a faithful quotient the same step gives RN(a/b).
-// Both last steps are Markstein's (P. Markstein, Computation of elementary
-// functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990).
-// They hold while nothing leaves the normal range: divisor_inside and
-// quotient_inside; what they refuse, a caller divides.
-__device__ __forceinline__ double recip_fast(double b) {
+// The Newton-Raphson iteration with fused multiply-adds, its last step and the
+// quotient's are Markstein's (P. Markstein, Computation of elementary functions
+// on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990).  They hold
+// while nothing leaves the normal range: divisor_inside and quotient_inside; what
+// they refuse, a caller divides.
+__device__ __forceinline__ double recip_start(double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    const double e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, __fma_rn(e, e, e), y);
-    return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+    return y;
+}
+__device__ __forceinline__ double newton_step(double b, double y) { return __fma_rn(y, __fma_rn(-b, y, 1.0), y); }
+__device__ __forceinline__ double recip_fast(double b) {
+    return newton_step(b, newton_step(b, newton_step(b, recip_start(b))));
 }
 __device__ __forceinline__ double quotient_fast(double a, double b, double y) {
     const double q0 = a * y;
@@ -52,7 +55,7 @@ __device__ __forceinline__ bool divisor_inside(double b) {    // 2^-100 <= |b| <
     const unsigned hi = (unsigned)__double2hiint(b);
     return (hi & 0x7fffffffu) - 0x39b00000u < 0x0c900000u && ((hi | 0xfff00000u) & (unsigned)__double2loint(b)) != ~0u;
 }
-__device__ __forceinline__ bool quotient_inside(double a) {   // a zero, or 2^-895 <= |a| < 2^770
+__device__ __forceinline__ bool quotient_inside(double a) {   // a zero, or 2^-895 <= |a| < 2^769 (1 + 2^-20)
     const unsigned hi = (unsigned)__double2hiint(a) & 0x7fffffffu;
     return hi - 0x08000000u <= 0x68000000u || (hi | (unsigned)__double2loint(a)) == 0u;
 }
