@@ -95,8 +95,8 @@ m2b_stage_kernel(const BatchInst<T>* __restrict__ inst, const int2* __restrict__
         }
         int tx, ty;
         unpack_tile(it, tx, ty);
-        m2_stage_tile<T, TX, TY, DEFER, GMODE, REC, NT, SPLIT>(s_inst.c, s_inst.buf[src], s_inst.buf[dst], s_inst.phi,
-                                                        nullptr, (T)dt[it.x], tx * TX, ty * TY, sm, s_inst.rec);
+        m2_stage_tile<T, TX, TY, DEFER, GMODE, REC, NT, SPLIT, false, sizeof(T) == 4 ? ESUM_BATCH : ESUM_FREE>(
+            s_inst.c, s_inst.buf[src], s_inst.buf[dst], s_inst.phi, nullptr, (T)dt[it.x], tx * TX, ty * TY, sm, s_inst.rec);
         __syncthreads();                            // shared tile buffers reused by the next tile
     }
 }
@@ -105,8 +105,7 @@ m2b_stage_kernel(const BatchInst<T>* __restrict__ inst, const int2* __restrict__
 // The FP32 stage as the register march of mhd2d_lane.cuh: a work item is an
 // instance, a segment length and four (strip, segment) pairs of that instance,
 // one to a warp, so that instances of one or two strips fill their CTAs too.
-// The tiles' bits (spelled-out sums: ESum; in 150 steps of the ensemble below one
-// update of some 10^9 differed in a last bit).  128 square instances of 64 to 256 cells a side (164 on
+// The tiles' bits (Stage32).  128 square instances of 64 to 256 cells a side (164 on
 // average) with gravity, first / second stage: tiles 317 / 343 us -> 185 / 222.
 // The instance's constants and planes are copied out of shared memory first:
 // read there they are loaded again in every row (192 / 235 us).

@@ -93,52 +93,73 @@ template <class T> constexpr size_t m2_stage_smem() { return StageGeom<T>::smem;
 // E, Bz, rho are updated.  Bx, By are the cell-centred stage-output B.
 // |J|^2 and the 5-point Laplacian of Bz of cell (i,j) of the stored state s,
 // whose own Bz is bzC (M2:640-668)
-// ES: the sums' products fused as in the tile kernels (FP32)
+// ES: the sums spelled out (FP32)
 template <class T, ESum ES = ESUM_FREE>
 __device__ __forceinline__ void joule_from(const M2Const<T>& c, T bzE, T bzW, T bzN, T bzS, T bzC, T dby, T dbx, T& J2,
                                            T& lap) {
-    J2 = divided<T>([&](auto& d) {
-        const T dBzdy = d.quot_by(bzN - bzS, c.two_dy, T(0.5) * c.inv_dy);
-        const T dBzdx = d.quot_by(bzE - bzW, c.two_dx, T(0.5) * c.inv_dx);
-        const T dBydx = d.quot_by(dby, c.dx, c.inv_dx);
-        const T dBxdy = d.quot_by(dbx, c.dy, c.inv_dy);
-        const T Jx = dBzdy, Jy = -dBzdx, Jz = dBydx - dBxdy;
-        if constexpr (ES == ESUM_GRID) return dot_spelled(Jy, Jy, Jx, Jx, Jz, Jz);
-        else if constexpr (ES == ESUM_BATCH) return dot_spelled(Jx, Jx, Jy, Jy, Jz, Jz);
-        else return Jx * Jx + Jy * Jy + Jz * Jz;
-    });
-    if constexpr (ES != ESUM_FREE) lap = fmaf(bzE - T(2) * bzC + bzW, c.idx2, __fmul_rn(bzN - T(2) * bzC + bzS, c.idy2));
-    else lap = (bzE - T(2) * bzC + bzW) * c.idx2 + (bzN - T(2) * bzC + bzS) * c.idy2;
+    if constexpr (ES != ESUM_FREE) {
+        const float Jx = __fmul_rn(bzN - bzS, 0.5f * c.inv_dy), Jy = -__fmul_rn(bzE - bzW, 0.5f * c.inv_dx);
+        const float Jz = fused_diff(dby, c.inv_dx, dbx, c.inv_dy);
+        J2 = ES == ESUM_GRID ? fused_dot(Jy, Jy, Jx, Jx, Jz, Jz) : fused_dot(Jx, Jx, Jy, Jy, Jz, Jz);
+        lap = fused_sum(fmaf(-2.0f, bzC, bzE) + bzW, c.idx2, fmaf(-2.0f, bzC, bzN) + bzS, c.idy2);
+    } else {
+        J2 = divided<T>([&](auto& d) {
+            const T dBzdy = d.quot_by(bzN - bzS, c.two_dy, T(0.5) * c.inv_dy);
+            const T dBzdx = d.quot_by(bzE - bzW, c.two_dx, T(0.5) * c.inv_dx);
+            const T dBydx = d.quot_by(dby, c.dx, c.inv_dx);
+            const T dBxdy = d.quot_by(dbx, c.dy, c.inv_dy);
+            const T Jx = dBzdy, Jy = -dBzdx, Jz = dBydx - dBxdy;
+            return Jx * Jx + Jy * Jy + Jz * Jz;
+        });
+        lap = (bzE - T(2) * bzC + bzW) * c.idx2 + (bzN - T(2) * bzC + bzS) * c.idy2;
+    }
 }
-template <class T>
+template <class T, ESum ES = ESUM_FREE>
 __device__ __forceinline__ void joule_terms(const M2Const<T>& c, const Fields<T>& s, int i, int j, T bzC, T& J2,
                                             T& lap) {
     const int P = c.pitch;
     const int iE = c.ax.cell(i + 1), iW = c.ax.cell(i - 1);
     const int jN = c.ay.cell(j + 1), jS = c.ay.cell(j - 1);
-    joule_from(c, s.Bz[(size_t)j * P + iE], s.Bz[(size_t)j * P + iW], s.Bz[(size_t)jN * P + i], s.Bz[(size_t)jS * P + i], bzC,
+    joule_from<T, ES>(c, s.Bz[(size_t)j * P + iE], s.Bz[(size_t)j * P + iW], s.Bz[(size_t)jN * P + i], s.Bz[(size_t)jS * P + i], bzC,
                s.by[(size_t)j * P + iE] - s.by[(size_t)j * P + i], s.bx[(size_t)jN * P + i] - s.bx[(size_t)j * P + i], J2, lap);
 }
 
 // eta J_z of an edge from the differences of By across it in x and of Bx in y (M2:565-575)
-template <class T> __device__ __forceinline__ T resistive_emf(const M2Const<T>& c, T dby, T dbx) {
-    return divided<T>([&](auto& d) {
-        const T dBydx = d.quot_by(dby, c.dx, c.inv_dx);
-        const T dBxdy = d.quot_by(dbx, c.dy, c.inv_dy);
-        return c.eta * (dBydx - dBxdy);
-    });
+template <class T, ESum ES = ESUM_FREE> __device__ __forceinline__ T resistive_emf(const M2Const<T>& c, T dby, T dbx) {
+    if constexpr (ES != ESUM_FREE) {
+        return __fmul_rn(c.eta, fused_diff(dby, c.inv_dx, dbx, c.inv_dy));
+    } else {
+        return divided<T>([&](auto& d) {
+            const T dBydx = d.quot_by(dby, c.dx, c.inv_dx);
+            const T dBxdy = d.quot_by(dbx, c.dy, c.inv_dy);
+            return c.eta * (dBydx - dBxdy);
+        });
+    }
 }
 
-template <class T>
+// the heating and the diffusion added to a cell, and its floors
+template <class T, ESum ES = ESUM_FREE>
+__device__ __forceinline__ void joule_add(const M2Const<T>& c, T dt, T J2, T lap, T& rho, T mx, T my, T mz, T& E, T& Bz, T Bx, T By) {
+    if constexpr (ES != ESUM_FREE) {
+        const float de = __fmul_rn(dt, c.eta);
+        E = fmaf(de, J2, E);
+        Bz = fmaf(de, lap, Bz);
+        Stage32<ES>::template floors<true>(c, rho, mx, my, mz, E, Bx, By, Bz);
+    } else {
+        E = E + dt * c.eta * J2;
+        Bz = Bz + dt * c.eta * lap;
+        floors(c, rho, mx, my, mz, E, Bx, By, Bz);
+    }
+}
+
+template <class T, ESum ES = ESUM_FREE>
 __device__ __forceinline__ void joule_cell(const M2Const<T>& c, const Fields<T>& s, int i, int j, T dt,
                                            T& rho, T mx, T my, T mz, T& E, T& Bz, T Bx, T By) {
     if (!c.resistive) return;
     const T bzC = Bz;
     T J2, lap;
-    joule_terms(c, s, i, j, bzC, J2, lap);
-    E = E + dt * c.eta * J2;
-    Bz = bzC + dt * c.eta * lap;
-    floors(c, rho, mx, my, mz, E, Bx, By, Bz);
+    joule_terms<T, ES>(c, s, i, j, bzC, J2, lap);
+    joule_add<T, ES>(c, dt, J2, lap, rho, mx, my, mz, E, Bz, Bx, By);
 }
 
 // ---------------------------------------------------------------------------
@@ -211,8 +232,9 @@ __device__ __forceinline__ void joule_cell_comp(const M2Const<T>& c, const Field
 // with comp_add.  The physics (primitives, slopes, fluxes, EMFs) reads the
 // FP32 values only, computed exactly as without KAHAN, so neighbouring tiles
 // see identical primitives.  Needs kahan_smem_extra<T>(TX*TY) more bytes.
+// ES: FP32 without KAHAN, the forms of Stage32.
 template <class T, int TX_, int TY_, bool DEFER, int GMODE, bool REC = false, int NT_ = TX_ * TY_,
-          bool SPLIT_ = false, bool KAHAN = false>
+          bool SPLIT_ = false, bool KAHAN = false, ESum ES = ESUM_FREE>
 __device__ __forceinline__ void m2_stage_tile(const M2Const<T>& c, const Fields<T>& in, const Fields<T>& out,
                                               const T* __restrict__ ga, const T* __restrict__ gb, const T dt,
                                               const int i0, const int j0, T* sm, T* const* rec = nullptr,
@@ -256,8 +278,10 @@ __device__ __forceinline__ void m2_stage_tile(const M2Const<T>& c, const Fields<
                 own_lo[3 * NC + o] = lin.mz[q]; own_lo[4 * NC + o] = l4; own_lo[5 * NC + o] = l5;
             }
         }
-        if (DEFER) joule_cell(c, in, ci, cj, dt, rho, mx, my, mz, E, Bz, Bx, By);
-        const Prim<T> W = to_prim(c, rho, mx, my, mz, E, Bx, By, Bz);
+        if (DEFER) joule_cell<T, ES>(c, in, ci, cj, dt, rho, mx, my, mz, E, Bz, Bx, By);
+        Prim<T> W;
+        if constexpr (ES != ESUM_FREE) W = Stage32<ES>::to_prim(c, rho, mx, my, mz, E, Bx, By, Bz);
+        else W = to_prim(c, rho, mx, my, mz, E, Bx, By, Bz);
         s_r[k] = W.r; s_u[k] = W.u; s_v[k] = W.v; s_w[k] = W.w;
         s_P[k] = W.P; s_bx[k] = W.bx; s_by[k] = W.by; s_bz[k] = W.bz;
         if (!KAHAN && mine) {
@@ -352,7 +376,7 @@ __device__ __forceinline__ void m2_stage_tile(const M2Const<T>& c, const Fields<
         const int cj = c.ay.cell(j0 + r);
         Flux<T> F;
         if constexpr (std::is_same<T, float>::value) {
-            F = hlld_x2(c, face_pair(ridx(f - 1, r), sidx(f - 1, r), ridx(f, r), sidx(f, r), false),
+            F = hlld_x2<ES>(c, face_pair(ridx(f - 1, r), sidx(f - 1, r), ridx(f, r), sidx(f, r), false),
                         in.bx[(size_t)cj * P + gi]);
         } else {
             const Prim<T> WL = face_state(ridx(f - 1, r), sidx(f - 1, r), false, T(1));
@@ -370,7 +394,7 @@ __device__ __forceinline__ void m2_stage_tile(const M2Const<T>& c, const Fields<
         const int ci = c.ax.cell(i0 + col);
         Flux<T> Gf;
         if constexpr (std::is_same<T, float>::value) {
-            Gf = hlld_x2(c, face_pair(ridx(col, g - 1), sidx(col, g - 1), ridx(col, g), sidx(col, g), true),
+            Gf = hlld_x2<ES>(c, face_pair(ridx(col, g - 1), sidx(col, g - 1), ridx(col, g), sidx(col, g), true),
                          in.by[(size_t)gj * P + ci]);
             const T t = Gf.f1; Gf.f1 = Gf.f2; Gf.f2 = t;   // hlld_y's swap back
         } else {
@@ -426,7 +450,7 @@ __device__ __forceinline__ void m2_stage_tile(const M2Const<T>& c, const Fields<
             const int cj = c.ay.cell(je), cjm = c.ay.cell(je - 1);
             const T dby = in.by[(size_t)je * P + ci] - in.by[(size_t)je * P + cim];
             const T dbx = in.bx[(size_t)cj * P + ie] - in.bx[(size_t)cjm * P + ie];
-            res = resistive_emf(c, dby, dbx);
+            res = resistive_emf<T, ES>(c, dby, dbx);
         }
         ez[k] = ideal + res;
     }
@@ -449,11 +473,12 @@ __device__ __forceinline__ void m2_stage_tile(const M2Const<T>& c, const Fields<
     {
         const int kxL = (ty + 1) * (TX + 1) + tx;
         const int kgD = ty * (TX + 2) + tx + 1, kgU = kgD + (TX + 2);
+        auto dF = [&](int m) { return fx[m * NFX + kxL + 1] - fx[m * NFX + kxL]; };
+        auto dG = [&](int m) { return gy[m * NGY + kgU] - gy[m * NGY + kgD]; };
         T d[7];
 #pragma unroll
         for (int m = 0; m < 7; m++)
-            d[m] = -(fx[m * NFX + kxL + 1] - fx[m * NFX + kxL]) * c.inv_dx -
-                   (gy[m * NGY + kgU] - gy[m * NGY + kgD]) * c.inv_dy;
+            d[m] = -dF(m) * c.inv_dx - dG(m) * c.inv_dy;
         const int kc = ridx(tx, ty);
         if constexpr (KAHAN) {
             comp_add(rho, lrho, dt * d[0]);
@@ -463,6 +488,18 @@ __device__ __forceinline__ void m2_stage_tile(const M2Const<T>& c, const Fields<
             comp_add(E, lE, dt * d[4]);
             comp_add(Bz, lBz, dt * d[6]);
             floors_comp(c, rho, lrho, mx, my, mz, E, lE, s_bx[kc], s_by[kc], Bz);
+        } else if constexpr (ES != ESUM_FREE) {
+            using S = Stage32<ES>;
+            rho = S::update(c, rho, dt, dF(0), dG(0));
+            mx = S::update(c, mx, dt, dF(1), dG(1));
+            my = S::update(c, my, dt, dF(2), dG(2));
+            mz = S::update(c, mz, dt, dF(3), dG(3));
+            E = S::update(c, E, dt, dF(4), dG(4));
+            Bz = S::update(c, Bz, dt, dF(6), dG(6));
+            if (REC) {
+                rec[0][q] = rho; rec[1][q] = mx; rec[2][q] = my; rec[3][q] = mz; rec[4][q] = E; rec[5][q] = Bz;
+            }
+            S::floors(c, rho, mx, my, mz, E, s_bx[kc], s_by[kc], Bz);
         } else {
             rho += dt * d[0];
             mx += dt * d[1];
@@ -498,6 +535,11 @@ __device__ __forceinline__ void m2_stage_tile(const M2Const<T>& c, const Fields<
         if (gi == c.nx - 1) lout.bx[q + 1] = l1;
         lout.by[q] = l2;
         if (gj == c.ny - 1) lout.by[q + P] = l3;
+    } else if constexpr (ES != ESUM_FREE) {
+        bxL = Stage32<ES>::ct(in.bx[q], -dtdy, e01 - e00);
+        bxR = Stage32<ES>::ct(in.bx[q + 1], -dtdy, e11 - e10);
+        byD = Stage32<ES>::ct(in.by[q], dtdx, e10 - e00);
+        byU = Stage32<ES>::ct(in.by[q + P], dtdx, e11 - e01);
     } else {
         bxL = in.bx[q] + -(dtdy) * (e01 - e00);
         bxR = in.bx[q + 1] + -(dtdy) * (e11 - e10);
@@ -522,6 +564,11 @@ __device__ __forceinline__ void m2_stage_tile(const M2Const<T>& c, const Fields<
             const T py = -(phi[(size_t)jN * P + gi] - phi[(size_t)jS * P + gi]);
             gxq = divided<T>([&](auto& d) { return d.quot_by(px, c.two_dx, T(0.5) * c.inv_dx); });
             gyq = divided<T>([&](auto& d) { return d.quot_by(py, c.two_dy, T(0.5) * c.inv_dy); });
+        }
+        if constexpr (ES != ESUM_FREE) {
+            Stage32<ES>::kick(c, dt, gxq, gyq, rho, mx, my, mz, E, T(0.5) * (bxL + bxR), T(0.5) * (byD + byU), Bz);
+            out.rho[q] = rho; out.mx[q] = mx; out.my[q] = my; out.mz[q] = mz; out.E[q] = E; out.Bz[q] = Bz;
+            return;
         }
         const Vel<T> V = velocity(vmax(rho, tiny_pos<T>()), mx, my, T(0.0));
         const T u = V.u, v = V.v;
@@ -553,7 +600,8 @@ m2_stage_kernel(const M2Const<T> c, const Fields<T> in, const Fields<T> out, con
     constexpr int TX = StageTile<T>::TX, TY = StageTile<T>::TY;
     if (active && *active == 0) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    m2_stage_tile<T, TX, TY, DEFER, GMODE, false, StageTile<T>::NT, StageTile<T>::SPLIT>(
+    m2_stage_tile<T, TX, TY, DEFER, GMODE, false, StageTile<T>::NT, StageTile<T>::SPLIT, false,
+                  sizeof(T) == 4 ? ESUM_GRID : ESUM_FREE>(
         c, in, out, ga, gb, (T)(*dtp), blockIdx.x * TX, blockIdx.y * TY, reinterpret_cast<T*>(smem_raw));
 }
 

@@ -12,8 +12,7 @@
 // shuffles and its global loads; the strip's halo lanes cost 32/28, the rows a
 // segment starts with 2 rows of x faces and 4 of primitives.
 //
-// Same expressions as the tile kernel and the same contractions, so the same
-// bits (the energy flux needs them spelled out: ESum).
+// Same functions as the tile kernel (Stage32, hlld_x2, joule_from), so the same bits.
 // That is kept on purpose: some FP32 runs amplify a last bit to 1e-3 of a weak
 // field within a hundred steps, so a cheaper HLLD with shared reciprocals (598 /
 // 715 us below) would have changed their results.
@@ -120,16 +119,14 @@ __device__ __forceinline__ void m2_lane_segment(LaneKeep& keep, const M2Const<fl
             const float zC = Bz;
             float J2, lap;
             joule_from<float, ES>(c, zE, zW, raw.zN, zS, zC, yE - raw.y0, raw.bN - raw.b0, J2, lap);
-            E = E + dt * c.eta * J2;
-            Bz = zC + dt * c.eta * lap;
-            floors(c, rho, mx, my, mz, E, Bx, By, Bz);
+            joule_add<float, ES>(c, dt, J2, lap, rho, mx, my, mz, E, Bz, Bx, By);
         }
         if (DEFER) zS = raw.Bz;
         const float rb0 = raw.b0, rb1 = raw.b1, ry0 = raw.y0, rphi = GMODE == GRAV_PHI ? raw.phi : 0.f;
         if (r <= j1) load(r + 1);
         keep.u[slot][0][tid] = make_float4(rho, mx, my, mz);
         keep.u[slot][1][tid] = make_float4(E, Bz, Bx, By);
-        const Prim<float> W = to_prim(c, rho, mx, my, mz, E, Bx, By, Bz);
+        const Prim<float> W = Stage32<ES>::to_prim(c, rho, mx, my, mz, E, Bx, By, Bz);
         // ---- slopes of row r - 1 along y; its face states ----
         const Row7 dp{W.r - w.r, W.u - w.u, W.v - w.v, W.w - w.w, W.P - w.P, W.bz - w.bz, W.bx - w.bx};
         if (r >= j0) {
@@ -173,18 +170,18 @@ __device__ __forceinline__ void m2_lane_segment(LaneKeep& keep, const M2Const<fl
                 float res = 0.f;
                 if (c.resistive) {
                     const float dby = bnY - lane_up(bnY), dbx = bn - bnx;
-                    res = resistive_emf(c, dby, dbx);
+                    res = resistive_emf<float, ES>(c, dby, dbx);
                 }
                 ez = ideal + res;
                 // CT of the row's lower y faces (M2:819-830)
-                byN = bnY + dtdx * (lane_down(ez) - ez);
+                byN = Stage32<ES>::ct(bnY, dtdx, lane_down(ez) - ez);
                 if (cell && (row < j1 || row == ny)) out.by[(size_t)row * P + gi] = byN;
             }
             // ---- finish the cells of row r - 2: update, floors, CT, gravity, store (M2:750-779, 807-832) ----
             if (r >= j0 + 2) {
                 const int jr = r - 2;
                 const size_t qb = (size_t)jr * P;
-                const float bxN = bnx + -(dtdy) * (ez - Ez);
+                const float bxN = Stage32<ES>::ct(bnx, -dtdy, ez - Ez);
                 const float bxR = lane_down(bxN);
                 float pE1 = 0.f, pW1 = 0.f;
                 if (GMODE == GRAV_PHI) { pE1 = lane_down(ph2); pW1 = lane_up(ph2); }
@@ -196,14 +193,14 @@ __device__ __forceinline__ void m2_lane_segment(LaneKeep& keep, const M2Const<fl
                     float u0 = a.x, u1 = a.y, u2 = a.z, u3 = a.w, u4 = b.x, u5 = b.y;
                     const float bxc = b.z, byc = b.w;
                     const float4 f0 = keep.f[0][tid], f1 = keep.f[1][tid], f2 = keep.f[2][tid];
-                    auto d = [&](float dF, float up, float G) { return -dF * c.inv_dx - (up - G) * c.inv_dy; };
-                    u0 += dt * d(f0.x, Gy[0], f1.z);
-                    u1 += dt * d(f0.y, Gy[1], f1.w);
-                    u2 += dt * d(f0.z, Gy[2], f2.x);
-                    u3 += dt * d(f0.w, Gy[3], f2.y);
-                    u4 += dt * d(f1.x, Gy[4], f2.z);
-                    u5 += dt * d(f1.y, Gy[6], f2.w);
-                    floors(c, u0, u1, u2, u3, u4, bxc, byc, u5);
+                    using S = Stage32<ES>;
+                    u0 = S::update(c, u0, dt, f0.x, Gy[0] - f1.z);
+                    u1 = S::update(c, u1, dt, f0.y, Gy[1] - f1.w);
+                    u2 = S::update(c, u2, dt, f0.z, Gy[2] - f2.x);
+                    u3 = S::update(c, u3, dt, f0.w, Gy[3] - f2.y);
+                    u4 = S::update(c, u4, dt, f1.x, Gy[4] - f2.z);
+                    u5 = S::update(c, u5, dt, f1.y, Gy[6] - f2.w);
+                    S::floors(c, u0, u1, u2, u3, u4, bxc, byc, u5);
                     if (GMODE != GRAV_NONE && c.gravity_on) {
                         float gxq, gyq;
                         if (GMODE == GRAV_ARRAYS) {
@@ -212,12 +209,7 @@ __device__ __forceinline__ void m2_lane_segment(LaneKeep& keep, const M2Const<fl
                             gxq = -(pE1 - pW1) * (0.5f * c.inv_dx);
                             gyq = -(ph1 - ph3) * (0.5f * c.inv_dy);
                         }
-                        const float ir = 1.0f / vmax(u0, tiny_pos<float>());
-                        const float u = u1 * ir, v = u2 * ir;
-                        u1 += dt * u0 * gxq;
-                        u2 += dt * u0 * gyq;
-                        u4 += dt * u0 * (u * gxq + v * gyq);
-                        floors(c, u0, u1, u2, u3, u4, 0.5f * (bxN + bxR), 0.5f * (byD + byN), u5);
+                        S::kick(c, dt, gxq, gyq, u0, u1, u2, u3, u4, 0.5f * (bxN + bxR), 0.5f * (byD + byN), u5);
                     }
                     out.rho[q] = u0; out.mx[q] = u1; out.my[q] = u2; out.mz[q] = u3; out.E[q] = u4; out.Bz[q] = u5;
                 }

@@ -403,30 +403,101 @@ __device__ __forceinline__ Prim<float> lane_y(const Prim2& S) {
     return Prim<float>{S.r.y, S.u.y, S.v.y, S.w.y, S.P.y, S.bx.y, S.by.y, S.bz.y};
 }
 
-// Some sums of two products, in the energy flux and the Joule heating, can be
-// fused in two ways, and which one the compiler takes depends on the order in which
-// the kernel around forms the operands.  The register march (mhd2d_lane.cuh) has them
-// spelled out as they are in the tile kernel of a single grid or in that of a batch,
-// which differ in the internal and kinetic energy and in J^2, so that a grid has the
-// same bits in either form.
+// The FP32 stage with its multiply-adds spelled out.  A sum of products can be
+// fused in several ways (a x + b y with either product inside, a quotient's last
+// product with the sum that follows), and which one the compiler takes depends on
+// the kernel around it.  The stage comes as tiles and as a register march
+// (mhd2d_lane.cuh), chosen by the size of a grid or of a whole ensemble, which must
+// not show in a result: both are built from the functions below, so that they have
+// the same bits whatever the compiler does.  ESUM_FREE leaves the choice to the
+// compiler (the compensated stage, the column march, the adjoint's recomputation);
+// ESUM_GRID and ESUM_BATCH are the forms that a single grid's and an ensemble's
+// tiles were compiled to before they were written down, which differ in the
+// internal and kinetic energy, in J^2 and in the floor after the Joule sub-step.
 enum ESum { ESUM_FREE, ESUM_GRID, ESUM_BATCH };
 
-// a x + b y + c z, spelled out as above
-__device__ __forceinline__ float dot_spelled(float a, float x, float b, float y, float c, float z) {
-    return fmaf(c, z, fmaf(a, x, __fmul_rn(b, y)));
+// a x + b y and a x - b y with the first product inside the multiply-add, a x + b y + c z on top of the former
+__device__ __forceinline__ float fused_sum(float a, float x, float b, float y) { return fmaf(a, x, __fmul_rn(b, y)); }
+__device__ __forceinline__ float fused_diff(float a, float x, float b, float y) { return fmaf(a, x, -__fmul_rn(b, y)); }
+__device__ __forceinline__ float fused_dot(float a, float x, float b, float y, float c, float z) {
+    return fmaf(c, z, fused_sum(a, x, b, y));
 }
-// energy flux of ideal_flux in that form; vB: its v . B
-template <ESum ES>
-__device__ __forceinline__ float energy_flux(const M2Const<float>& c, const Prim<float>& W, float& vB) {
-    const float B2 = fmaf(W.bz, W.bz, fmaf(W.by, W.by, __fmul_rn(W.bx, W.bx)));
-    const float k = dot_spelled(W.u, W.u, W.v, W.v, W.w, W.w);
-    vB = dot_spelled(W.u, W.bx, W.v, W.by, W.w, W.bz);
-    const float ig = 1.0f / c.gm1, hr = __fmul_rn(0.5f, W.r);
-    const float ek = ES == ESUM_GRID ? fmaf(W.P, ig, __fmul_rn(hr, k)) : fmaf(hr, k, __fmul_rn(W.P, ig));
-    const float E = fmaf(0.5f, B2, ek);
-    const float pt = fmaf(0.5f, B2, W.P);
-    return fmaf(E + pt, W.u, -__fmul_rn(W.bx, vB));
-}
+
+template <ESum ES> struct Stage32 {
+    // velocity, twice the kinetic energy over rho, B^2 and gamma - 1 times what they leave of E
+    struct Cell { float u, v, w, hr, k, B2, P; };
+    static __device__ __forceinline__ Cell cell(const M2Const<float>& c, float rho, float mx, float my, float mz, float E, float Bx,
+                                                float By, float Bz) {
+        Cell q;
+        const float ir = 1.0f / rho;
+        q.u = __fmul_rn(mx, ir); q.v = __fmul_rn(my, ir); q.w = __fmul_rn(mz, ir);
+        q.hr = __fmul_rn(0.5f, rho);
+        q.k = fused_dot(q.u, q.u, q.v, q.v, q.w, q.w);
+        q.B2 = fused_dot(Bx, Bx, By, By, Bz, Bz);
+        q.P = __fmul_rn(c.gm1, fmaf(-0.5f, q.B2, fmaf(-q.hr, q.k, E)));
+        return q;
+    }
+    static __device__ __forceinline__ Prim<float> to_prim(const M2Const<float>& c, float rho, float mx, float my, float mz, float E,
+                                                          float Bx, float By, float Bz) {
+        rho = vmax(rho, c.floor_rho);
+        const Cell q = cell(c, rho, mx, my, mz, E, Bx, By, Bz);
+        Prim<float> W;
+        W.r = rho; W.u = q.u; W.v = q.v; W.w = q.w; W.P = q.P < c.floor_P ? c.floor_P : q.P;
+        W.bx = Bx; W.by = By; W.bz = Bz;
+        return W;
+    }
+    // floors after the update or the gravity kick, or (JOULE) after the Joule sub-step
+    template <bool JOULE = false>
+    static __device__ __forceinline__ void floors(const M2Const<float>& c, float& rho, float mx, float my, float mz, float& E, float Bx,
+                                                  float By, float Bz) {
+        rho = vmax(rho, c.floor_rho);
+        const Cell q = cell(c, rho, mx, my, mz, E, Bx, By, Bz);
+        const float ig = 1.0f / c.gm1;
+        float low;
+        if constexpr (JOULE) {
+            const float e = ES == ESUM_GRID ? fused_sum(q.hr, q.k, 0.5f, q.B2) : fused_sum(0.5f, q.B2, q.hr, q.k);
+            low = __fadd_rn(e, __fmul_rn(c.floor_P, ig));
+        } else {
+            low = fmaf(c.floor_P, ig, fused_sum(0.5f, q.B2, q.hr, q.k));
+        }
+        if (q.P < c.floor_P) E = low;
+    }
+    // ideal_flux; vB: its v . B
+    static __device__ __forceinline__ Flux<float> flux(const M2Const<float>& c, const Prim<float>& W, float& vB) {
+        const float ru = __fmul_rn(W.r, W.u);
+        const float B2 = fused_dot(W.by, W.by, W.bx, W.bx, W.bz, W.bz);
+        const float k = fused_dot(W.u, W.u, W.v, W.v, W.w, W.w);
+        vB = fused_dot(W.u, W.bx, W.v, W.by, W.w, W.bz);
+        const float ig = 1.0f / c.gm1, hr = __fmul_rn(0.5f, W.r);
+        const float ek = ES == ESUM_GRID ? fused_sum(W.P, ig, hr, k) : fused_sum(hr, k, W.P, ig);
+        const float E = fmaf(0.5f, B2, ek), pt = fmaf(0.5f, B2, W.P);
+        Flux<float> F;
+        F.f0 = ru;
+        F.f1 = __fsub_rn(fmaf(ru, W.u, pt), __fmul_rn(W.bx, W.bx));
+        F.f2 = fused_diff(ru, W.v, W.bx, W.by);
+        F.f3 = fused_diff(ru, W.w, W.bx, W.bz);
+        F.f4 = fused_diff(__fadd_rn(E, pt), W.u, W.bx, vB);
+        F.f5 = fused_diff(W.u, W.by, W.v, W.bx);
+        F.f6 = fused_diff(W.u, W.bz, W.w, W.bx);
+        return F;
+    }
+    // flux divergence from the differences of the x and the y fluxes
+    static __device__ __forceinline__ float update(const M2Const<float>& c, float u, float dt, float dF, float dG) {
+        return fmaf(dt, fused_diff(-dF, c.inv_dx, dG, c.inv_dy), u);
+    }
+    // a face's B from the difference of its edges' EMFs; r: dt / dy, signed
+    static __device__ __forceinline__ float ct(float b, float r, float de) { return fmaf(r, de, b); }
+    // gravity kick (M2:602-629) and its floors
+    static __device__ __forceinline__ void kick(const M2Const<float>& c, float dt, float gx, float gy, float& rho, float& mx, float& my,
+                                                float mz, float& E, float Bx, float By, float Bz) {
+        const float ir = 1.0f / vmax(rho, tiny_pos<float>());
+        const float u = __fmul_rn(mx, ir), v = __fmul_rn(my, ir), dr = __fmul_rn(dt, rho);
+        mx = fmaf(dr, gx, mx);
+        my = fmaf(dr, gy, my);
+        E = fmaf(dr, fused_sum(u, gx, v, gy), E);
+        floors(c, rho, mx, my, mz, E, Bx, By, Bz);
+    }
+};
 
 template <ESum ES = ESUM_FREE>
 __device__ __forceinline__ Flux<float> hlld_x2(const M2Const<float>& c, Prim2 S, const float Bn) {
@@ -448,12 +519,12 @@ __device__ __forceinline__ Flux<float> hlld_x2(const M2Const<float>& c, Prim2 S,
     const float SL = fminf(um.x, um.y);
     const float SR = fmaxf(up.x, up.y);
     auto flux_of = [&](const Prim<float>& W) {
-        Flux<float> F = ideal_flux(c, W);
         if constexpr (ES != ESUM_FREE) {
             float vB;
-            F.f4 = energy_flux<ES>(c, W, vB);
+            return Stage32<ES>::flux(c, W, vB);
+        } else {
+            return ideal_flux(c, W);
         }
-        return F;
     };
     if (0.0f <= SL) return flux_of(lane_x(S));
     if (0.0f >= SR) return flux_of(lane_y(S));
@@ -470,6 +541,17 @@ __device__ __forceinline__ Flux<float> hlld_x2(const M2Const<float>& c, Prim2 S,
         const float inv = 1.0f / (SR - SL);
         const float s2 = SL * SR;
         Flux<float> F;
+        if constexpr (ES != ESUM_FREE) {
+            auto hll = [&](float l, float r, float d) { return __fmul_rn(fmaf(s2, d, fused_diff(SR, l, SL, r)), inv); };
+            F.f0 = hll(FL.f0, FR.f0, R.r - L.r);
+            F.f1 = hll(FL.f1, FR.f1, FR.f0 - FL.f0);
+            F.f2 = hll(FL.f2, FR.f2, fused_diff(R.r, R.v, L.r, L.v));
+            F.f3 = hll(FL.f3, FR.f3, fused_diff(R.r, R.w, L.r, L.w));
+            F.f4 = hll(FL.f4, FR.f4, E.y - E.x);
+            F.f5 = hll(FL.f5, FR.f5, R.by - L.by);
+            F.f6 = hll(FL.f6, FR.f6, R.bz - L.bz);
+            return F;
+        }
         F.f0 = (SR * FL.f0 - SL * FR.f0 + s2 * (R.r - L.r)) * inv;
         F.f1 = (SR * FL.f1 - SL * FR.f1 + s2 * (R.r * R.u - L.r * L.u)) * inv;
         F.f2 = (SR * FL.f2 - SL * FR.f2 + s2 * (R.r * R.v - L.r * L.v)) * inv;
@@ -492,7 +574,9 @@ __device__ __forceinline__ Flux<float> hlld_x2(const M2Const<float>& c, Prim2 S,
     }
     const float2 SmM = psub(SLR, pbc(SM));     // S - SM of each side
     const float2 rst = pk(rsd.x / SmM.x, rsd.y / SmM.y);
-    const float pts = pt.x + rsd.x * (SM - S.u.x);
+    float pts;
+    if constexpr (ES != ESUM_FREE) pts = fmaf(rsd.x, __fsub_rn(SM, S.u.x), pt.x);
+    else pts = pt.x + rsd.x * (SM - S.u.x);
     const float bn2 = Bn * Bn;
     const float2 dLR = pfma(rsd, SmM, pbc(-bn2));
     const float2 num = pfma(rsd, sLR, pbc(-bn2));
@@ -524,24 +608,38 @@ __device__ __forceinline__ Flux<float> hlld_x2(const M2Const<float>& c, Prim2 S,
     } else {
         const float sgn = (Bn >= 0.0f) ? 1.0f : -1.0f;
         const float id2 = 1.0f / (sq.x + sq.y);
-        vs = (sq.x * vs2.x + sq.y * vs2.y + (Bys2.y - Bys2.x) * sgn) * id2;
-        ws = (sq.x * ws2.x + sq.y * ws2.y + (Bzs2.y - Bzs2.x) * sgn) * id2;
-        Bys = (sq.x * Bys2.y + sq.y * Bys2.x + sq.x * sq.y * (vs2.y - vs2.x) * sgn) * id2;
-        Bzs = (sq.x * Bzs2.y + sq.y * Bzs2.x + sq.x * sq.y * (ws2.y - ws2.x) * sgn) * id2;
+        if constexpr (ES != ESUM_FREE) {
+            const float sxy = __fmul_rn(sq.x, sq.y);
+            vs = __fmul_rn(fmaf(Bys2.y - Bys2.x, sgn, fused_sum(sq.x, vs2.x, sq.y, vs2.y)), id2);
+            ws = __fmul_rn(fmaf(Bzs2.y - Bzs2.x, sgn, fused_sum(sq.x, ws2.x, sq.y, ws2.y)), id2);
+            Bys = __fmul_rn(fmaf(__fmul_rn(sxy, vs2.y - vs2.x), sgn, fused_sum(sq.x, Bys2.y, sq.y, Bys2.x)), id2);
+            Bzs = __fmul_rn(fmaf(__fmul_rn(sxy, ws2.y - ws2.x), sgn, fused_sum(sq.x, Bzs2.y, sq.y, Bzs2.x)), id2);
+        } else {
+            vs = (sq.x * vs2.x + sq.y * vs2.y + (Bys2.y - Bys2.x) * sgn) * id2;
+            ws = (sq.x * ws2.x + sq.y * ws2.y + (Bzs2.y - Bzs2.x) * sgn) * id2;
+            Bys = (sq.x * Bys2.y + sq.y * Bys2.x + sq.x * sq.y * (vs2.y - vs2.x) * sgn) * id2;
+            Bzs = (sq.x * Bzs2.y + sq.y * Bzs2.x + sq.x * sq.y * (ws2.y - ws2.x) * sgn) * id2;
+        }
     }
-    Flux<float> F = ideal_flux(c, W);
-    float Es;
     if constexpr (ES != ESUM_FREE) {
         float vBw;
-        F.f4 = energy_flux<ES>(c, W, vBw);
-        const float vBs = dot_spelled(SM, Bn, vs, Bys, ws, Bzs);
-        const float wW = fmaf(ptW, W.u, -__fmul_rn(Bn, vBw)), wS = fmaf(pts, SM, -__fmul_rn(Bn, vBs));
-        Es = (fmaf(Sw - W.u, EW, -wW) + wS) / (Sw - SM);
-    } else {
-        const float vBs = SM * Bn + vs * Bys + ws * Bzs;
-        const float vBw = W.u * W.bx + W.v * W.by + W.w * W.bz;
-        Es = ((Sw - W.u) * EW - (ptW * W.u - Bn * vBw) + (pts * SM - Bn * vBs)) / (Sw - SM);
+        Flux<float> F = Stage32<ES>::flux(c, W, vBw);
+        const float vBs = fused_dot(SM, Bn, vs, Bys, ws, Bzs);
+        const float wW = fused_diff(ptW, W.u, Bn, vBw), wS = fused_diff(pts, SM, Bn, vBs);
+        const float num = __fadd_rn(fmaf(Sw - W.u, EW, -wW), wS), rec = 1.0f / __fsub_rn(Sw, SM);   // E* = num rec
+        F.f0 = fmaf(Sw, __fsub_rn(rs, W.r), F.f0);
+        F.f1 = fmaf(Sw, fused_diff(rs, SM, W.r, W.u), F.f1);
+        F.f2 = fmaf(Sw, fused_diff(rs, vs, W.r, W.v), F.f2);
+        F.f3 = fmaf(Sw, fused_diff(rs, ws, W.r, W.w), F.f3);
+        F.f4 = fmaf(Sw, fmaf(num, rec, -EW), F.f4);
+        F.f5 = fmaf(Sw, __fsub_rn(Bys, W.by), F.f5);
+        F.f6 = fmaf(Sw, __fsub_rn(Bzs, W.bz), F.f6);
+        return F;
     }
+    Flux<float> F = ideal_flux(c, W);
+    const float vBs = SM * Bn + vs * Bys + ws * Bzs;
+    const float vBw = W.u * W.bx + W.v * W.by + W.w * W.bz;
+    const float Es = ((Sw - W.u) * EW - (ptW * W.u - Bn * vBw) + (pts * SM - Bn * vBs)) / (Sw - SM);
     F.f0 = F.f0 + Sw * (rs - W.r);
     F.f1 = F.f1 + Sw * (rs * SM - W.r * W.u);
     F.f2 = F.f2 + Sw * (rs * vs - W.r * W.v);
