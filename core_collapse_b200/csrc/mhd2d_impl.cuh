@@ -95,18 +95,19 @@ cudaError_t M2Launch<T>::prepare(int nx, int ny) {
             }
         }
     }
-    constexpr int CW = (sizeof(T) == 8) ? 2 : 4;
-    const int smem_row = (int)(sizeof(Cplx<T>) * (size_t)fft_line_slots(nx)) * fft_lines_per_cta(nx, ny);
-    const int smem_col = (int)(sizeof(Cplx<T>) * (size_t)fft_col_stride(ny) * CW);
-    if (smem_row <= 227 * 1024 && smem_col <= 227 * 1024) {  // larger lines are rejected by the solver set-up
-#define CC_FFT_ATTR(RB)                                          \
-        CC_ATTR((fft_rows_fwd_kernel<T, RB>), smem_row)          \
-        CC_ATTR((fft_rows_inv_kernel<T, RB>), smem_row)          \
-        CC_ATTR((fft_cols_solve_kernel<T, CW, RB>), smem_col)
-        CC_FFT_ATTR(2)
-        CC_FFT_ATTR(3)
-        CC_FFT_ATTR(4)
+    if constexpr (sizeof(T) == 8) {
+        const int smem_row = (int)(sizeof(Cplx<T>) * (size_t)fft_line_slots(nx)) * fft_lines_per_cta(nx, ny);
+        const int smem_col = (int)(sizeof(Cplx<T>) * (size_t)fft_col_stride(ny) * FFT_CW);
+        if (smem_row <= 227 * 1024 && smem_col <= 227 * 1024) {  // larger lines are rejected by the solver set-up
+#define CC_FFT_ATTR(RB)                                      \
+            CC_ATTR((fft_rows_fwd_kernel<T, RB>), smem_row)  \
+            CC_ATTR((fft_rows_inv_kernel<T, RB>), smem_row)  \
+            CC_ATTR((fft_cols_solve_kernel<T, FFT_CW, RB>), smem_col)
+            CC_FFT_ATTR(2)
+            CC_FFT_ATTR(3)
+            CC_FFT_ATTR(4)
 #undef CC_FFT_ATTR
+        }
     }
 #undef CC_ATTR
     return cudaSuccess;
@@ -309,30 +310,34 @@ cudaError_t M2Launch<T>::fft_solve(const T* rho, int pitch, const double* rho_pa
                                    int logny, const Cplx<T>* twx_f, const Cplx<T>* twx_i, const Cplx<T>* twy_f,
                                    const Cplx<T>* twy_i, double Lx, double Ly, double G, Cplx<T>* A, T* phi,
                                    const int* active, cudaStream_t s) {
-    constexpr int CW = (sizeof(T) == 8) ? 2 : 4;  // 32-byte column strips
-    const int rx = fft_stages_per_pass(nx), ry = fft_stages_per_pass(ny);
-    const int lines = fft_lines_per_cta(nx, ny), nt_row = fft_threads(nx, lines, rx);
-    const size_t smem_row = sizeof(Cplx<T>) * (size_t)fft_line_slots(nx) * lines;
-    const size_t smem_col = sizeof(Cplx<T>) * (size_t)fft_col_stride(ny) * CW;
-    const double ncell = (double)nx * (double)ny;
-    cudaError_t e;
+    if constexpr (sizeof(T) != 8) {
+        return cudaErrorNotSupported;   // fft32_solve
+    } else {
+        const int rx = fft_stages_per_pass(nx), ry = fft_stages_per_pass(ny);
+        const int lines = fft_lines_per_cta(nx, ny), nt_row = fft_threads(nx, lines, rx);
+        const size_t smem_row = sizeof(Cplx<T>) * (size_t)fft_line_slots(nx) * lines;
+        const size_t smem_col = sizeof(Cplx<T>) * (size_t)fft_col_stride(ny) * FFT_CW;
+        const double ncell = (double)nx * (double)ny;
+        // one group of elements to a thread (fft_turn)
+        const int ncolblk = (nx + FFT_CW - 1) / FFT_CW, nt_col = fft_threads(ny, FFT_CW, ry);
+        if (FFT_CW * ny >> ry > nt_col) return cudaErrorInvalidValue;
+        cudaError_t e;
 #define CC_FFT_BY(R, LAUNCH) \
-    switch (R) {             \
-        case 2: { constexpr int RB = 2; LAUNCH; } break; \
-        case 3: { constexpr int RB = 3; LAUNCH; } break; \
-        default: { constexpr int RB = 4; LAUNCH; } break; \
-    }                        \
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    CC_FFT_BY(rx, (fft_rows_fwd_kernel<T, RB><<<ny / lines, nt_row, smem_row, s>>>(
-                      rho, pitch, rho_part, RED_BLOCKS, ncell, A, nx, lognx, lines, twx_f, active)))
-    // one group of elements to a thread (fft_turn)
-    const int ncolblk = (nx + CW - 1) / CW, nt_col = fft_threads(ny, CW, ry);
-    CC_FFT_BY(ry, (fft_cols_solve_kernel<T, CW, RB><<<ncolblk, nt_col, smem_col, s>>>(A, nx, ny, logny, twy_f, twy_i, Lx,
-                                                                                      Ly, G, active)))
-    CC_FFT_BY(rx, (fft_rows_inv_kernel<T, RB><<<ny / lines, nt_row, smem_row, s>>>(A, nx, lognx, lines, twx_i, phi, pitch,
-                                                                                   active)))
+        switch (R) {             \
+            case 2: { constexpr int RB = 2; LAUNCH; } break; \
+            case 3: { constexpr int RB = 3; LAUNCH; } break; \
+            default: { constexpr int RB = 4; LAUNCH; } break; \
+        }                        \
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        CC_FFT_BY(rx, (fft_rows_fwd_kernel<T, RB><<<ny / lines, nt_row, smem_row, s>>>(
+                          rho, pitch, rho_part, RED_BLOCKS, ncell, A, nx, lognx, lines, twx_f, active)))
+        CC_FFT_BY(ry, (fft_cols_solve_kernel<T, FFT_CW, RB><<<ncolblk, nt_col, smem_col, s>>>(A, nx, ny, logny, twy_f, twy_i,
+                                                                                              Lx, Ly, G, active)))
+        CC_FFT_BY(rx, (fft_rows_inv_kernel<T, RB><<<ny / lines, nt_row, smem_row, s>>>(A, nx, lognx, lines, twx_i, phi, pitch,
+                                                                                       active)))
 #undef CC_FFT_BY
-    return cudaSuccess;
+        return cudaSuccess;
+    }
 }
 
 template <class T>

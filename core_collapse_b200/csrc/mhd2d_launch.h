@@ -60,7 +60,7 @@ template <class T> struct M2Launch {
     static cudaError_t derived(const M2Const<T>& c, const Fields<T>& st, double* out, cudaStream_t s);
     static cudaError_t pack_in(const double* src, T* dst, int w, int h, int pitch, cudaStream_t s);
     static cudaError_t pack_out(const T* src, double* dst, int w, int h, int pitch, cudaStream_t s);
-    // spectral solve: rho (pitched T) -> phi (pitched T); A: nx*ny complex work
+    // FP64 spectral solve (FP32: fft32_solve), T = double only: rho (pitched T) -> phi (pitched T); A: nx*ny complex work
     static cudaError_t fft_solve(const T* rho, int pitch, const double* rho_part, int nx, int ny, int lognx,
                                  int logny, const Cplx<T>* twx_f, const Cplx<T>* twx_i, const Cplx<T>* twy_f,
                                  const Cplx<T>* twy_i, double Lx, double Ly, double G, Cplx<T>* A, T* phi,

@@ -12,9 +12,10 @@
 // columns-then-rows so that the column inverse fuses with the spectral
 // multiply (rounding differs at the 1e-16 level; stated in the tests).
 //
-// Red-black SOR (the GPU ordering of M2:207-223 / EH:335-368): a persistent
-// cooperative kernel, one grid barrier per colour, deterministic FP64 mean
-// removal after each sweep (applied lazily, see sor_rb_kernel), optional
+// Red-black SOR (the GPU ordering of M2:207-223 / EH:335-368): grids up to about
+// 360^2 inside one thread-block cluster (sor_cluster_kernel), larger ones in a
+// persistent cooperative kernel with one grid barrier per colour (sor_rb_kernel);
+// deterministic FP64 mean removal after each sweep (applied lazily), optional
 // residual test.
 #pragma once
 #include <cooperative_groups.h>
@@ -117,7 +118,7 @@ __device__ __forceinline__ void fft_first(Cplx<T>* a, int LS, int n, int logn, i
     __syncthreads();
 }
 
-// Stages h0 .. 8 h0 within shared memory, or out of it through st(line, index, x) (LAST, 16 h0 = n).
+// R stages from h0 on within shared memory, or out of it through st(line, index, x) (LAST, 2^R h0 = n).
 template <class T, int R, bool IL, bool LAST, class ST>
 __device__ __forceinline__ void fft_next(Cplx<T>* a, int LS, int n, int lines, int h0, const Cplx<T>* __restrict__ tw, ST st) {
     constexpr int M = 1 << R;
@@ -166,10 +167,10 @@ __device__ __forceinline__ void fft_lines(Cplx<T>* a, int LS, int n, int logn, i
     fft_next<T, RB, IL, true>(a, LS, n, lines, h0, tw, st);
 }
 
-// the kernels below run on at most FFT_NT threads
-constexpr int FFT_NT = 512;
+// the kernels below run on at most FFT_NT threads; the column pass takes FFT_CW columns (32 bytes of a row) a CTA
+constexpr int FFT_NT = 512, FFT_CW = 2;
 
-// lines of an n-point transform to a CTA (of `total`), and its threads: one per group of 16
+// lines of an n-point transform to a CTA (of `total`), and its threads: one per group of 2^RB
 __host__ __device__ inline int fft_lines_per_cta(int n, int total) {
     const int l = n >= 512 ? 1 : 512 / n;
     return l < total ? l : total;
