@@ -65,6 +65,7 @@ constexpr int SOR_NT = 1024;
 // beyond which the whole chip is as fast), a row the pairs of a CTA, and the
 // pairs the blocks of sor_rb_kernel one to a thread (an odd nx can exceed them
 // by a few), whose sums it repeats.
+constexpr size_t SOR_CL_MAX_SMEM = 224 * 1024;
 struct SorClusterPlan { int V, nc; size_t smem; };
 static SorClusterPlan sor_cluster_plan(const SorArgs& a) {
     SorClusterPlan p{0, 0, 0};
@@ -75,14 +76,15 @@ static SorClusterPlan sor_cluster_plan(const SorArgs& a) {
     if (M > (a.nx * a.ny / 2 + SOR_NT - 1) / SOR_NT * SOR_NT) return p;
     const int S = (nb + SOR_CL_MAXC - 1) / SOR_CL_MAXC * SOR_NT, V = S / SOR_CL_NT;
     const size_t smem = sor_cluster_smem(S, half, nb);
-    if (V > SOR_CL_MAXV || half > S || smem > 224 * 1024) return p;
+    if (V > SOR_CL_MAXV || half > S || smem > SOR_CL_MAX_SMEM) return p;
     p.V = V; p.nc = (M + S - 1) / S; p.smem = smem;
     return p;
 }
 
 template <int V> static cudaError_t launch_sor_cluster(const SorArgs& a, const SorClusterPlan& p, cudaStream_t s, bool* done) {
     const void* fn = (const void*)sor_cluster_kernel<V>;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+    // the limit is the device's, for every handle and captured graph: what the largest grid may take, not this one
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOR_CL_MAX_SMEM);
     if (e == cudaSuccess && p.nc > 8) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute at[1];
