@@ -163,7 +163,7 @@ template <class T> struct Mhd2d : Mhd2dBase {
         c.resistive = (p.eta > 0.0) ? 1 : 0;
         plane = (size_t)P * (ny + 1);
         march_rows = default_march_rows(nx, ny);
-        CC_CUDA(M2Launch<T>::prepare(nx, ny));
+        CC_CUDA(M2Launch<T>::prepare());
 
         if (p.compensated && sizeof(T) != 4)
             return fail(h, CC_ERR_UNSUPPORTED, "the compensated update is an option of the FP32 path");

@@ -112,7 +112,7 @@ template <class T> struct Ns2d : Ns2dBase {
                 return fail(h, CC_ERR_UNSUPPORTED, "FP32 FFT Poisson supports Nx, Ny <= 8192");
         }
         CC_CUDA(NSLaunch<T>::prepare());
-        CC_CUDA(M2Launch<T>::prepare(nx, ny));
+        CC_CUDA(M2Launch<T>::prepare());
         CC_CUDA(cudaMalloc(&block, sizeof(T) * plane * 12));
         CC_CUDA(cudaMemsetAsync(block, 0, sizeof(T) * plane * 12, st()));
         T* b = reinterpret_cast<T*>(block);

@@ -1,5 +1,7 @@
 // Definitions of M2Launch<T>; included once per precision TU.
 #pragma once
+#include <algorithm>
+
 #include "mhd2d_lane.cuh"
 #include "mhd2d_launch.h"
 
@@ -25,8 +27,20 @@ inline int grid_for(size_t n, int nt, int cap) {
 }
 }  // namespace
 
+// The most that size(n) takes over the transform lengths n = lo, 2 lo .. hi (what does not fit an SM is
+// refused by the set-up of a solver or never taken).
+template <class F> size_t largest_line(int lo, int hi, F size) {
+    size_t m = 0;
+    for (int n = lo; n <= hi; n *= 2)
+        if (size(n) <= 227 * 1024) m = std::max(m, (size_t)size(n));
+    return m;
+}
+
+// A function's limit belongs to the whole device and serves every handle, so it is
+// set to what the longest accepted line needs, whatever handle asks: a limit of a
+// handle's own grid would refuse the launches of one with longer lines.
 template <class T>
-cudaError_t M2Launch<T>::prepare(int nx, int ny) {
+cudaError_t M2Launch<T>::prepare() {
     const int smem = (int)m2_stage_smem<T>();
     cudaError_t e;
 #define CC_ATTR(K, BYTES)                                                                              \
@@ -59,55 +73,46 @@ cudaError_t M2Launch<T>::prepare(int nx, int ny) {
         CC_ATTR((m2_stage_comp_kernel<T, true, GRAV_PHI>), smem_c)
     }
     if constexpr (sizeof(T) == 4) {
-        if (nx >= 2 && ny >= 2) {
-            const int row = (int)(sizeof(float2) * (size_t)fft32_line(nx));
-            const int col = (int)(sizeof(float2) * (size_t)fft32_line(ny)) * fft32_cw(ny);
-            if (row <= 227 * 1024 && col <= 227 * 1024) {
-                CC_ATTR((f32_rows_fwd_kernel<T, false>), row)
-                CC_ATTR((f32_rows_fwd_kernel<T, true>), row)
-                CC_ATTR((f32_rows_inv_kernel<T, 0>), row)
-                CC_ATTR((f32_rows_inv_kernel<T, 2>), row)
-                CC_ATTR((f32_rows_inv_kernel<T, 4>), row)
-                CC_ATTR((f32_rows_inv_kernel<T, 8>), row)
-                CC_ATTR((f32_rows_inv_kernel<T, 16>), row)
-                CC_ATTR((f32_cols_rk_kernel<16, 16>), col)
-                CC_ATTR((f32_cols_rk_kernel<8, 2>), col)
-                CC_ATTR((f32_cols_rk_kernel<4, 4>), col)
-                CC_ATTR((f32_cols_rk_kernel<2, 8>), col)
-                CC_ATTR((f32_cols_rk_kernel<1, 16>), col)
-                CC_ATTR((f32_cols_rk_kernel<1, 2>), col)
-                if (ny >= 256) {
-                    const int tsm = (int)fft32_cols_tma_smem(fft32_cw(ny), ny);
-                    if (tsm <= 227 * 1024) {
-                        CC_ATTR((f32_cols_tma_kernel<16, 16>), tsm)
-                        CC_ATTR((f32_cols_tma_kernel<8, 2>), tsm)
-                        CC_ATTR((f32_cols_tma_kernel<4, 4>), tsm)
-                        CC_ATTR((f32_cols_tma_kernel<2, 8>), tsm)
-                        CC_ATTR((f32_cols_tma_kernel<1, 16>), tsm)
-                        CC_ATTR((f32_cols_tma_kernel<1, 2>), tsm)
-                    }
-                }
-                CC_ATTR(f32_cols_solve_kernel<1>, col)
-                CC_ATTR(f32_cols_solve_kernel<2>, col)
-                CC_ATTR(f32_cols_solve_kernel<4>, col)
-                CC_ATTR(f32_cols_solve_kernel<8>, col)
-                CC_ATTR(f32_cols_solve_kernel<16>, col)
-            }
-        }
+        const int row = (int)largest_line(2, FFT32_MAXN, [](int n) { return sizeof(float2) * (size_t)fft32_line(n); });
+        const int col = (int)largest_line(2, FFT32_MAXN, [](int n) { return sizeof(float2) * (size_t)fft32_line(n) * fft32_cw(n); });
+        const int tsm = (int)largest_line(256, FFT32_MAXN, [](int n) { return (size_t)fft32_cols_tma_smem(fft32_cw(n), n); });
+        CC_ATTR((f32_rows_fwd_kernel<T, false>), row)
+        CC_ATTR((f32_rows_fwd_kernel<T, true>), row)
+        CC_ATTR((f32_rows_inv_kernel<T, 0>), row)
+        CC_ATTR((f32_rows_inv_kernel<T, 2>), row)
+        CC_ATTR((f32_rows_inv_kernel<T, 4>), row)
+        CC_ATTR((f32_rows_inv_kernel<T, 8>), row)
+        CC_ATTR((f32_rows_inv_kernel<T, 16>), row)
+        CC_ATTR((f32_cols_rk_kernel<16, 16>), col)
+        CC_ATTR((f32_cols_rk_kernel<8, 2>), col)
+        CC_ATTR((f32_cols_rk_kernel<4, 4>), col)
+        CC_ATTR((f32_cols_rk_kernel<2, 8>), col)
+        CC_ATTR((f32_cols_rk_kernel<1, 16>), col)
+        CC_ATTR((f32_cols_rk_kernel<1, 2>), col)
+        CC_ATTR((f32_cols_tma_kernel<16, 16>), tsm)
+        CC_ATTR((f32_cols_tma_kernel<8, 2>), tsm)
+        CC_ATTR((f32_cols_tma_kernel<4, 4>), tsm)
+        CC_ATTR((f32_cols_tma_kernel<2, 8>), tsm)
+        CC_ATTR((f32_cols_tma_kernel<1, 16>), tsm)
+        CC_ATTR((f32_cols_tma_kernel<1, 2>), tsm)
+        CC_ATTR(f32_cols_solve_kernel<1>, col)
+        CC_ATTR(f32_cols_solve_kernel<2>, col)
+        CC_ATTR(f32_cols_solve_kernel<4>, col)
+        CC_ATTR(f32_cols_solve_kernel<8>, col)
+        CC_ATTR(f32_cols_solve_kernel<16>, col)
     }
     if constexpr (sizeof(T) == 8) {
-        const int smem_row = (int)(sizeof(Cplx<T>) * (size_t)fft_line_slots(nx)) * fft_lines_per_cta(nx, ny);
-        const int smem_col = (int)(sizeof(Cplx<T>) * (size_t)fft_col_stride(ny) * FFT_CW);
-        if (smem_row <= 227 * 1024 && smem_col <= 227 * 1024) {  // larger lines are rejected by the solver set-up
-#define CC_FFT_ATTR(RB)                                      \
-            CC_ATTR((fft_rows_fwd_kernel<T, RB>), smem_row)  \
-            CC_ATTR((fft_rows_inv_kernel<T, RB>), smem_row)  \
-            CC_ATTR((fft_cols_solve_kernel<T, FFT_CW, RB>), smem_col)
-            CC_FFT_ATTR(2)
-            CC_FFT_ATTR(3)
-            CC_FFT_ATTR(4)
+        // (a short line's rows go several to a CTA, at most 512 points of them)
+        const int row = (int)largest_line(512, 1 << 14, [](int n) { return sizeof(Cplx<T>) * (size_t)fft_line_slots(n); });
+        const int col = (int)largest_line(2, 1 << 14, [](int n) { return sizeof(Cplx<T>) * (size_t)fft_col_stride(n) * FFT_CW; });
+#define CC_FFT_ATTR(RB)                             \
+        CC_ATTR((fft_rows_fwd_kernel<T, RB>), row)  \
+        CC_ATTR((fft_rows_inv_kernel<T, RB>), row)  \
+        CC_ATTR((fft_cols_solve_kernel<T, FFT_CW, RB>), col)
+        CC_FFT_ATTR(2)
+        CC_FFT_ATTR(3)
+        CC_FFT_ATTR(4)
 #undef CC_FFT_ATTR
-        }
     }
 #undef CC_ATTR
     return cudaSuccess;

@@ -28,7 +28,7 @@ inline double stage_lane_us(long ctas, int rows) {
 
 template <class T> struct M2Launch {
     // raise the dynamic shared-memory limits of the kernels (once per device, before any launch or capture)
-    static cudaError_t prepare(int nx, int ny);
+    static cudaError_t prepare();
     static cudaError_t stage(const M2Const<T>& c, const Fields<T>& in, const Fields<T>& out, bool defer, int gmode,
                              const T* ga, const T* gb, const double* dt, const int* active, cudaStream_t s);
     static cudaError_t average(const M2Const<T>& c, const Fields<T>& un, const Fields<T>& s2, const Fields<T>& out,

@@ -73,7 +73,7 @@ int device_scratch(double** base) {
     if (!d.ready) {
         void* ptr = nullptr;
         if (cudaGetSymbolAddress(&ptr, cc_noalloc_scratch) != cudaSuccess || ptr == nullptr) return CC_ERR_CUDA;
-        if (M2Launch<double>::prepare((int)NA_MAX_SIDE, (int)NA_MAX_SIDE) != cudaSuccess) return CC_ERR_CUDA;
+        if (M2Launch<double>::prepare() != cudaSuccess) return CC_ERR_CUDA;
         d.base = static_cast<double*>(ptr);
         d.ready = true;
     }
