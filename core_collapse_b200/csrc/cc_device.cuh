@@ -104,6 +104,12 @@ template <class T, bool PLAIN> struct Div {
 #endif
         return quot(a, b, y);
     }
+    // a / b by a constant of the grid whose reciprocal y the host has rounded; FP32 divides (quot_by: a y, which
+    // rounds differently)
+    __host__ __device__ __forceinline__ T quot_grid(T a, T b, T y) {
+        if constexpr (sizeof(T) == 4) return a / b;
+        else return quot_by(a, b, y);
+    }
     // a / b, a denominator of its own
     __host__ __device__ __forceinline__ T div(T a, T b) {
         if constexpr (FAST64) return quot(a, b, recip(b));

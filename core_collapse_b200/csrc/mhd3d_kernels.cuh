@@ -62,20 +62,6 @@ __device__ __forceinline__ T bz_cc3(const M3Const<T>& c, const T* bz, int i, int
     return T(0.5) * (bzf3(c, bz, i, j, k) + bzf3(c, bz, i, j, k + 1));
 }
 
-// Joule heating E += dt eta |J|^2 of cell (i,j,k) (add_joule_heating, M3:652-692)
-template <class T>
-__device__ __forceinline__ T joule3(const M3Const<T>& c, const Fields3<T>& s, int i, int j, int k, T dt) {
-    const T dBzdy = (bz_cc3(c, s.bz, i, j + 1, k) - bz_cc3(c, s.bz, i, j - 1, k)) / c.two_dy;
-    const T dBydz = (by_cc3(c, s.by, i, j, k + 1) - by_cc3(c, s.by, i, j, k - 1)) / c.two_dz;
-    const T dBxdz = (bx_cc3(c, s.bx, i, j, k + 1) - bx_cc3(c, s.bx, i, j, k - 1)) / c.two_dz;
-    const T dBzdx = (bz_cc3(c, s.bz, i + 1, j, k) - bz_cc3(c, s.bz, i - 1, j, k)) / c.two_dx;
-    const T dBydx = (by_cc3(c, s.by, i + 1, j, k) - by_cc3(c, s.by, i - 1, j, k)) / c.two_dx;
-    const T dBxdy = (bx_cc3(c, s.bx, i, j + 1, k) - bx_cc3(c, s.bx, i, j - 1, k)) / c.two_dy;
-    const T Jx = dBzdy - dBydz, Jy = dBxdz - dBzdx, Jz = dBydx - dBxdy;
-    const T J2 = Jx * Jx + Jy * Jy + Jz * Jz;
-    return dt * c.eta * J2;
-}
-
 // Cell-centred B planes of a state (bx_cc3, by_cc3, bz_cc3 of every cell),
 // written once before a Joule pass so that the pass reads 12 stored values per
 // cell instead of forming them from 24 face loads.  The values are the same
@@ -83,8 +69,8 @@ __device__ __forceinline__ T joule3(const M3Const<T>& c, const Fields3<T>& s, in
 // the stored value at its mapped cell, the cell map being idempotent.
 template <class T> struct Bcc3 { T* x; T* y; T* z; };
 
-// Joule heating of cell (i,j,k) in the box (add_joule_heating, M3:652-692),
-// as joule3 with the cell-centred B read from b
+// Joule heating dt eta |J|^2 of cell (i,j,k) in the box (add_joule_heating,
+// M3:652-692), the cell-centred B read from b
 template <class T>
 __device__ __forceinline__ T joule3_cc(const M3Const<T>& c, const Bcc3<T>& b, int i, int j, int k, T dt) {
     auto at = [&](const T* f, int a, int bb, int d) { return f[c.idx(a, bb, d)]; };
@@ -95,9 +81,9 @@ __device__ __forceinline__ T joule3_cc(const M3Const<T>& c, const Bcc3<T>& b, in
     const T bx_y = at(b.y, ip, j, k) - at(b.y, im, j, k), by_x = at(b.x, i, jp, k) - at(b.x, i, jm, k);
     const T hx = T(0.5) * c.inv_dx, hy = T(0.5) * c.inv_dy, hz = T(0.5) * c.inv_dz;
     const T J2 = divided<T>([&](auto& d) {
-        const T dBzdy = d.quot_by(by_z, c.two_dy, hy), dBydz = d.quot_by(bz_y, c.two_dz, hz);
-        const T dBxdz = d.quot_by(bz_x, c.two_dz, hz), dBzdx = d.quot_by(bx_z, c.two_dx, hx);
-        const T dBydx = d.quot_by(bx_y, c.two_dx, hx), dBxdy = d.quot_by(by_x, c.two_dy, hy);
+        const T dBzdy = d.quot_grid(by_z, c.two_dy, hy), dBydz = d.quot_grid(bz_y, c.two_dz, hz);
+        const T dBxdz = d.quot_grid(bz_x, c.two_dz, hz), dBzdx = d.quot_grid(bx_z, c.two_dx, hx);
+        const T dBydx = d.quot_grid(bx_y, c.two_dx, hx), dBxdy = d.quot_grid(by_x, c.two_dy, hy);
         const T Jx = dBzdy - dBydz, Jy = dBxdz - dBzdx, Jz = dBydx - dBxdy;
         return Jx * Jx + Jy * Jy + Jz * Jz;
     });
@@ -331,6 +317,15 @@ __global__ void __launch_bounds__(256) m3_update_kernel(const M3Const<T> c, cons
     }
 }
 
+// eta (d1 / h1 - d2 / h2), h1 and h2 grid spacings with the reciprocals i1 and i2
+template <class T>
+__device__ __forceinline__ T m3_resistive_emf(const M3Const<T>& c, T d1, T h1, T i1, T d2, T h2, T i2) {
+    return divided<T>([&](auto& d) {
+        const T a = d.quot_grid(d1, h1, i1), b = d.quot_grid(d2, h2, i2);
+        return c.eta * (a - b);
+    });
+}
+
 // Edge EMFs (M3:879-939): Balsara-Spicer average of the four face EMFs plus
 // eta J from cell-centred B differences; Ex at (i, jf, kf), Ey at (if, j, kf),
 // Ez at (if, jf, k).  EdgeColumn marches one (i, j) edge column in k,
@@ -367,14 +362,6 @@ template <class T> struct EdgeColumn {
         }
     }
 
-    // eta (d1 / h1 - d2 / h2)
-    __device__ __forceinline__ T curl(T d1, T h1, T i1, T d2, T h2, T i2) const {
-        return divided<T>([&](auto& d) {
-            const T a = d.quot_by(d1, h1, i1), b = d.quot_by(d2, h2, i2);
-            return c.eta * (a - b);
-        });
-    }
-
     // the three EMFs of plane k (0 where the edge does not exist), then advance
     __device__ __forceinline__ void step(int k, T& ex, T& ey, T& ez) {
         const int ck = c.az.cell(k), fk = c.az.face(k), fk1 = c.az.face(k + 1);
@@ -390,7 +377,7 @@ template <class T> struct EdgeColumn {
             T res = T(0.0);
             if (res_on) {
                 const T dbz = T(0.5) * (bz0 + bz1) - T(0.5) * (bz0s + bz1s), dby = by_k - by_p;
-                res = curl(dbz, c.dy, c.inv_dy, dby, c.dz, c.inv_dz);
+                res = m3_resistive_emf(c, dbz, c.dy, c.inv_dy, dby, c.dz, c.inv_dz);
             }
             ex = ideal + res;
         }
@@ -399,7 +386,7 @@ template <class T> struct EdgeColumn {
             T res = T(0.0);
             if (res_on) {
                 const T dbx = bx_k - bx_p, dbz = T(0.5) * (bz0 + bz1) - T(0.5) * (bz0w + bz1w);
-                res = curl(dbx, c.dz, c.inv_dz, dbz, c.dx, c.inv_dx);
+                res = m3_resistive_emf(c, dbx, c.dz, c.inv_dz, dbz, c.dx, c.inv_dx);
             }
             ey = ideal + res;
         }
@@ -409,7 +396,7 @@ template <class T> struct EdgeColumn {
             T res = T(0.0);
             if (res_on) {
                 const T dby = by_k - byc(cim, ck), dbx = bx_k - bxc(cjm, ck);
-                res = curl(dby, c.dx, c.inv_dx, dbx, c.dy, c.inv_dy);
+                res = m3_resistive_emf(c, dby, c.dx, c.inv_dx, dbx, c.dy, c.inv_dy);
             }
             ez = ideal + res;
         }
