@@ -43,14 +43,14 @@ int default_march_rows(int nx, int ny) {
     return (int)rows;
 }
 // The FP32 stage of a grid: rows per warp of the register march, or 0 where the
-// tiles are faster by the counts of mhd2d_launch.h.  The march has to be 8%
-// ahead, for their errors; the line lies near 500^2.  Steps without gravity,
+// tiles are faster by the counts of mhd2d_launch.h (asked: the best march all the
+// same).  The march has to be 8% ahead, for their errors; the line lies near 500^2.  Steps without gravity,
 // tiles and best march: 256^2 33.8 and 35.6 us, 384^2 42.9 either way, 512^2
 // 58.7 and 52.9, 900 x 700 103 and 96, 1003 x 777 122 and 99, 2048^2 588 and
 // 457, 4096^2 2252 and 1576.
-int lane_rows(int nx, int ny) {
+int lane_rows(int nx, int ny, bool asked = false) {
     auto div_up = [](long a, long b) { return (a + b - 1) / b; };
-    double best = 0.92 * stage_tiles_us(div_up(nx, 30) * div_up(ny, 15));
+    double best = asked ? 1e300 : 0.92 * stage_tiles_us(div_up(nx, 30) * div_up(ny, 15));
     int rows = 0;
     for (int seg = 2; seg <= 64; seg += 2) {
         if (div_up(ny, seg) > 65535) continue;   // grid.y
@@ -79,6 +79,7 @@ struct Mhd2dBase {
     virtual int set_clock(double t, long long steps) = 0;
     virtual const cc_mhd2d_params& params() const = 0;
     virtual int set_stage_kernel(int kind, int seg_rows) = 0;
+    virtual void get_stage_kernel(int* kind, int* seg_rows) = 0;
 };
 
 template <class T> struct Mhd2d : Mhd2dBase {
@@ -93,11 +94,11 @@ template <class T> struct Mhd2d : Mhd2dBase {
     bool comp = false;
     void* lblock = nullptr;
     Fields<T> lbuf[3];
-    // stage kernel: STAGE_AUTO (the register march in segments of lane_seg rows, or the tiles) until
-    // cc_mhd2d_set_stage_kernel asks for CC_STAGE_TILE or CC_STAGE_MARCH
-    static constexpr int STAGE_AUTO = -1;
-    int stage_kind = STAGE_AUTO;
-    int lane_seg = 0;     // 0: tiles (FP64, a compensated state, a small grid)
+    // stage kernel: what cc_mhd2d_set_stage_kernel asked for; CC_STAGE_AUTO: by the grid
+    int stage_kind = CC_STAGE_AUTO;
+    int lane_auto = 0;    // rows per warp of the register march that the grid picks; 0: tiles (FP64, a compensated
+                          // state, a small grid)
+    int lane_seg = 0;     // of the one that runs
     int march_rows = 0;   // 0: from the grid (init)
     int cur = 0;
     T* phi = nullptr;
@@ -168,7 +169,7 @@ template <class T> struct Mhd2d : Mhd2dBase {
         if (p.compensated && sizeof(T) != 4)
             return fail(h, CC_ERR_UNSUPPORTED, "the compensated update is an option of the FP32 path");
         comp = p.compensated != 0;
-        lane_seg = (sizeof(T) == 4 && !comp) ? lane_rows(nx, ny) : 0;
+        lane_seg = lane_auto = (sizeof(T) == 4 && !comp) ? lane_rows(nx, ny) : 0;
         CC_CUDA(cudaMalloc(&block, sizeof(T) * plane * 24));
         CC_CUDA(cudaMemsetAsync(block, 0, sizeof(T) * plane * 24, st()));
         for (int b = 0; b < 3; b++) {
@@ -413,6 +414,12 @@ template <class T> struct Mhd2d : Mhd2dBase {
 
     void count(int n) { h->perf.kernel_launches += n; }
 
+    // the stage kernel that runs
+    int stage_now() const {
+        if (stage_kind != CC_STAGE_AUTO) return stage_kind;
+        return lane_auto > 0 ? CC_STAGE_LANE : CC_STAGE_TILE;
+    }
+
     // one stage-kernel launch from buf[bi] to buf[bo], bracketed by CUDA events when profiling
     int stage(int bi, int bo, bool defer, int gmode, const T* ga, const T* gb) {
         cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -421,9 +428,10 @@ template <class T> struct Mhd2d : Mhd2dBase {
             CC_CUDA(cudaEventCreate(&e1));
             CC_CUDA(cudaEventRecord(e0, st()));
         }
-        if (stage_kind == STAGE_AUTO && lane_seg > 0)
+        const int kind = stage_now();
+        if (kind == CC_STAGE_LANE)
             CC_CUDA(M2Launch<T>::stage_lane(c, buf[bi], buf[bo], defer, gmode, ga, gb, dt_dev, active(), lane_seg, st()));
-        else if (stage_kind == CC_STAGE_MARCH)
+        else if (kind == CC_STAGE_MARCH)
             CC_CUDA(M2Launch<T>::stage_march(c, buf[bi], buf[bo], comp ? &lbuf[bi] : nullptr,
                                              comp ? &lbuf[bo] : nullptr, defer, gmode, ga, gb, dt_dev, active(),
                                              march_rows, st()));
@@ -576,14 +584,28 @@ template <class T> struct Mhd2d : Mhd2dBase {
     const cc_mhd2d_params& params() const override { return p; }
 
     int set_stage_kernel(int kind, int seg_rows) override {
-        if (kind != CC_STAGE_TILE && kind != CC_STAGE_MARCH) return fail(h, CC_ERR_ARG, "unknown stage kernel");
+        if (kind != CC_STAGE_TILE && kind != CC_STAGE_MARCH && kind != CC_STAGE_LANE && kind != CC_STAGE_AUTO)
+            return fail(h, CC_ERR_ARG, "unknown stage kernel");
         if (kind == CC_STAGE_MARCH && sizeof(T) != 4)
             return fail(h, CC_ERR_UNSUPPORTED, "the column-march stage kernel is an FP32 kernel");
+        if (kind == CC_STAGE_LANE && (sizeof(T) != 4 || comp))
+            return fail(h, CC_ERR_UNSUPPORTED, "the register march is a kernel of the uncompensated FP32 state");
         if (seg_rows < 0) return fail(h, CC_ERR_ARG, "seg_rows < 0");
+        if (kind == CC_STAGE_LANE) {
+            if (seg_rows > 0 && ((long)p.Ny + seg_rows - 1) / seg_rows > 65535) return fail(h, CC_ERR_ARG, "too many segments");
+            lane_seg = seg_rows > 0 ? seg_rows : lane_rows(p.Nx, p.Ny, true);
+            if (lane_seg == 0) return fail(h, CC_ERR_UNSUPPORTED, "the grid has too many rows for the register march");
+        }
+        if (kind == CC_STAGE_AUTO) lane_seg = lane_auto;
         stage_kind = kind;
-        march_rows = seg_rows > 0 ? seg_rows : default_march_rows(p.Nx, p.Ny);
+        march_rows = kind == CC_STAGE_MARCH && seg_rows > 0 ? seg_rows : default_march_rows(p.Nx, p.Ny);
         invalidate_graph();
         return CC_OK;
+    }
+
+    void get_stage_kernel(int* kind, int* seg_rows) override {
+        *kind = stage_now();
+        *seg_rows = *kind == CC_STAGE_LANE ? lane_seg : (*kind == CC_STAGE_MARCH ? march_rows : 0);
     }
 
     int derived(double* const* out) override {
@@ -804,6 +826,13 @@ int cc_mhd2d_set_stage_kernel(cc_handle* h, int kind, int seg_rows) {
     Mhd2dBase* m = m2(h);
     if (!m) return CC_ERR_ARG;
     return m->set_stage_kernel(kind, seg_rows);
+}
+
+int cc_mhd2d_get_stage_kernel(cc_handle* h, int* kind, int* seg_rows) {
+    Mhd2dBase* m = m2(h);
+    if (!m || !kind || !seg_rows) return CC_ERR_ARG;
+    m->get_stage_kernel(kind, seg_rows);
+    return CC_OK;
 }
 
 int cc_mhd2d_advance(cc_handle* h, int nsteps, double* t) {

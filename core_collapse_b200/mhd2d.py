@@ -211,10 +211,17 @@ class Mhd2dSolver:
         return tt.value
 
     def set_stage_kernel(self, kind: str, seg_rows: int = 0):
-        """"tile" (the default) or "march" (FP32 only), seg_rows 0: chosen from
-        the grid (cc_mhd2d_set_stage_kernel)."""
-        k = {"tile": L.CC_STAGE_TILE, "march": L.CC_STAGE_MARCH}[kind]
+        """"auto" (the default: by the grid), "tile", "lane" (the register march, FP32
+        only) or "march" (FP32 only); seg_rows 0: chosen from the grid
+        (cc_mhd2d_set_stage_kernel)."""
+        k = {"auto": L.CC_STAGE_AUTO, "tile": L.CC_STAGE_TILE, "lane": L.CC_STAGE_LANE, "march": L.CC_STAGE_MARCH}[kind]
         self._check(self._lib.cc_mhd2d_set_stage_kernel(self._h, k, int(seg_rows)))
+
+    def stage_kernel(self) -> tuple[str, int]:
+        """The stage kernel that runs ("tile", "lane" or "march") and its rows per segment (0: tiles)."""
+        k, rows = C.c_int(), C.c_int()
+        self._check(self._lib.cc_mhd2d_get_stage_kernel(self._h, C.byref(k), C.byref(rows)))
+        return {L.CC_STAGE_TILE: "tile", L.CC_STAGE_LANE: "lane", L.CC_STAGE_MARCH: "march"}[k.value], rows.value
 
     def set_stream(self, stream_ptr: int | None):
         """Issue work on a caller's cudaStream_t (e.g. torch's current stream)."""

@@ -256,16 +256,22 @@ int cc_mhd2d_advance(cc_handle* h, int nsteps, double* t);
 
 /* Choice of the stage kernel (no counterpart in the reference, whose
  * advance_stage M2:690-834 is one function): CC_STAGE_TILE, one CTA per tile of
- * cells with a recomputed halo (the only form for FP64), or CC_STAGE_MARCH,
- * FP32 only, a CTA per column strip that marches up a segment of seg_rows rows
- * carrying the rows below it (0: a length chosen from the grid so the segments
- * fill the GPU).  A handle that is not asked for one of them runs the tiles, or
- * on an uncompensated FP32 grid large enough to fill the GPU with them, warps
- * that march in registers.  All evaluate the same expressions; a tuning and
- * testing switch. */
+ * cells with a recomputed halo (the only form for FP64); CC_STAGE_LANE,
+ * uncompensated FP32 only, warps that march up segments of seg_rows rows in
+ * registers (0: a length chosen from the grid); CC_STAGE_MARCH, FP32 only, a CTA
+ * per column strip that marches up a segment of seg_rows rows carrying the rows
+ * below it (0: a length chosen from the grid so the segments fill the GPU); or
+ * CC_STAGE_AUTO, the default: the register march on an uncompensated FP32 grid
+ * large enough to fill the GPU with it, else the tiles.  All evaluate the same
+ * expressions, tiles and register march with the same bits; a tuning and testing
+ * switch. */
 #define CC_STAGE_TILE 0
 #define CC_STAGE_MARCH 1
+#define CC_STAGE_LANE 2
+#define CC_STAGE_AUTO 3
 int cc_mhd2d_set_stage_kernel(cc_handle* h, int kind, int seg_rows);
+/* The stage kernel that runs (CC_STAGE_TILE, _MARCH or _LANE) and its rows per segment (0: tiles). */
+int cc_mhd2d_get_stage_kernel(cc_handle* h, int* kind, int* seg_rows);
 
 /* Diagnostics of the resident state. */
 int cc_mhd2d_diagnostics(cc_handle* h, cc_diag* d);

@@ -58,10 +58,9 @@ def test_single_grid(regime, px, py):
     p = _params(regime, 700, 513, periodic_x=px, periodic_y=py, gravity_on=False)
     s0 = _state(regime, p, 1)
     out = []
-    for kind in (None, "tile"):
+    for kind in ("lane", "tile"):
         with Mhd2dSolver(p) as s:
-            if kind:
-                s.set_stage_kernel(kind)
+            s.set_stage_kernel(kind)
             s.upload(*s0)
             s.advance(3, 0.0)
             out.append(O.state_list(*s.download()))
@@ -73,10 +72,9 @@ def test_single_grid_gravity(regime):
     p = _params(regime, 1024, 512, periodic_x=True, periodic_y=True, gravity_on=True, poisson="fft")
     s0 = _state(regime, p, 2)
     out = []
-    for kind in (None, "tile"):
+    for kind in ("lane", "tile"):
         with Mhd2dSolver(p) as s:
-            if kind:
-                s.set_stage_kernel(kind)
+            s.set_stage_kernel(kind)
             s.upload(*s0)
             s.advance(3, 0.0)
             out.append(O.state_list(*s.download()))
