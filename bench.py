@@ -232,12 +232,16 @@ class ClockSampler:
 
 # ---------------------------------------------------------------- GPU arm
 
-def stage_capture(grid: int, key: str):
-    """A per-launch figure of the stage kernel (DRAM bytes, warp instructions)
-    from the committed ncu capture, scaled to the benchmark grid by cell count
-    (both grow with the cells: every tile reads its halo once and runs the same
-    work per cell)."""
-    f = ROOT / "profiles" / "stage_kernel_traffic.json"
+STAGE_KERNELS = {"tile": "m2_stage_kernel<float>", "lane": "m2_lane_kernel", "march": "m2_march_kernel<float>"}
+STAGE_CAPTURES = {"tile": "stage_kernel_traffic.json", "lane": "lane_kernel_traffic.json"}
+
+
+def stage_capture(kind: str, grid: int, key: str):
+    """A per-launch figure of the stage kernel that ran (DRAM bytes, warp
+    instructions) from its committed ncu capture, scaled to the benchmark grid
+    by cell count (both grow with the cells: every tile or strip reads its halo
+    once and runs the same work per cell); None for a kernel without one."""
+    f = ROOT / "profiles" / STAGE_CAPTURES.get(kind, "none")
     if not f.exists():
         return None
     d = json.loads(f.read_text())
@@ -247,15 +251,15 @@ def stage_capture(grid: int, key: str):
         return None
 
 
-def traffic_per_launch(grid: int):
-    return stage_capture(grid, "dram_bytes_per_launch")
+def traffic_per_launch(kind: str, grid: int):
+    return stage_capture(kind, grid, "dram_bytes_per_launch")
 
 
-def issue_roofline(grid: int, launch_ms: float, clk) -> dict | None:
+def issue_roofline(kind: str, grid: int, launch_ms: float, clk) -> dict | None:
     """The stage kernel's instruction-issue bound: its warp instructions per
     launch (ncu capture, scaled to the grid) over 148 SMs x 4 schedulers x one
     instruction per cycle at the SM clock sampled during the timed region."""
-    inst = stage_capture(grid, "warp_instructions_per_launch")
+    inst = stage_capture(kind, grid, "warp_instructions_per_launch")
     mhz = (clk or {}).get("sm_mhz") or (clk or {}).get("sm_max_mhz") or 1965
     if not inst or not launch_ms:
         return None
@@ -302,7 +306,7 @@ def run_ours(args) -> None:
         p = workload_params(n, precision)
         s = Mhd2dSolver(p)
         s.set_stream(stream.cuda_stream)
-        if precision == "fp32":
+        if precision == "fp32" and args.stage_kernel != "auto":
             s.set_stage_kernel(args.stage_kernel, args.march_rows)
         s.upload(U0, B0)
         s.advance(args.warmup, 0.0)
@@ -338,6 +342,7 @@ def run_ours(args) -> None:
     stage64_avg_ms = perf64["stage_ms"] / max(1, perf64["stage_launches"])
 
     d32 = s32.diagnostics()
+    stage_kind, stage_rows = s32.stage_kernel()
 
     # end to end through the C ABI with pinned host buffers, copies timed every
     # step: upload the state, one main-loop step, download the state
@@ -383,14 +388,13 @@ def run_ours(args) -> None:
                          "steps": e2e_steps, "api": "cc_mhd2d_upload + cc_mhd2d_advance(1) + cc_mhd2d_download, "
                                                     "pinned FP64 host"}},
         "fp32_over_fp64": value32 / value64,
-        "roofline": {"bound": "hbm", "kernel": ("m2_march_kernel<float>" if args.stage_kernel == "march"
-                                                else "m2_stage_kernel<float>") + " (one RK2 stage)",
+        "roofline": {"bound": "hbm", "kernel": STAGE_KERNELS[stage_kind] + " (one RK2 stage)", "stage_rows": stage_rows,
                      "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"], "peak_source": peaks["source"],
-                     "traffic": traffic_per_launch(n), "algorithmic_bytes_per_launch": stage_bytes,
+                     "traffic": traffic_per_launch(stage_kind, n), "algorithmic_bytes_per_launch": stage_bytes,
                      "launch_ms": stage_avg_ms,
                      "step_roofline_frac": STEP_WORDS * 4 * value32 / world / 1e9 / peaks["hbm_gbs"],
-                     "issue": issue_roofline(n, stage_avg_ms, clk)},
+                     "issue": issue_roofline(stage_kind, n, stage_avg_ms, clk)},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": h2d,
                 "steps": e2e_steps, "api": "cc_mhd2d_upload + cc_mhd2d_advance(1) + cc_mhd2d_download, pinned FP64 host"},
         "gpu_launches": perf32["kernel_launches"],
@@ -875,9 +879,9 @@ def main():
     ap.add_argument("--cpu-sample-grid", type=int, default=512)
     ap.add_argument("--cpu-steps", type=int, default=3)
     ap.add_argument("--no-cpu-baseline", action="store_true")
-    ap.add_argument("--stage-kernel", choices=["march", "tile"], default="tile",
-                    help="FP32 stage kernel of the headline run")
-    ap.add_argument("--march-rows", type=int, default=0, help="rows per march segment (0: from the grid)")
+    ap.add_argument("--stage-kernel", choices=["auto", "tile", "lane", "march"], default="auto",
+                    help="FP32 stage kernel of the headline run; auto: the one a handle picks by its grid")
+    ap.add_argument("--march-rows", type=int, default=0, help="rows per segment of the lane or march kernel (0: from the grid)")
     ap.add_argument("--skip-ladder", action="store_true")
     ap.add_argument("--ladder-steps", type=int, default=500)
     ap.add_argument("--ladder-grids", default="1024,4096")

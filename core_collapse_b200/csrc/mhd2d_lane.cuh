@@ -17,7 +17,7 @@
 // field within a hundred steps, so a cheaper HLLD with shared reciprocals (598 /
 // 715 us below) would have changed their results.
 //
-// Bound: issue (65% of the slots at 16 warps an SM; 128 registers allow no more,
+// Bound: issue (73% of the slots at 16 warps an SM; 128 registers allow no more,
 // and 20 warps at 96 registers spilled: 722 us) and the latency of a row's two
 // HLLD chains.  4096^2 with gravity, first / second stage of a step: tiles 1103
 // / 1156 us -> 661 / 778.  On the way: the potential carried instead of read at
