@@ -107,6 +107,8 @@ class BatchSolver:
         return {f: getattr(d, f) for f, _ in L.CcDiag._fields_}
 
     def autotune(self, reps: int = 5) -> tuple[int, float]:
+        """Times every stage candidate and keeps the fastest: (candidate, ms); the
+        candidate is set_shape's and info()["shape"]'s (cc_batch_autotune)."""
         shape, ms = C.c_int(), C.c_double()
         self._check(self._lib.cc_batch_autotune(self._h, reps, C.byref(shape), C.byref(ms)))
         return shape.value, ms.value

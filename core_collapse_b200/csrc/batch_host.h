@@ -123,9 +123,11 @@ template <class T> struct Batch : BatchBase {
     std::vector<int2*> swork;        // per stage shape
     std::vector<int> nswork;
     std::vector<int> sgrid;          // CTAs per candidate
-    // FP32: the register march, which runs unless it is the slower one by its
-    // count (nlwork 0) or by autotune, or a tile candidate was set
+    // FP32: the register march, candidate 2 NS of a batch whose work-list for it
+    // (nlwork) is not empty: there it is the faster one by its count and runs until
+    // autotune finds otherwise or a tile candidate is set
     int2* lwork = nullptr; int nlwork = 0;
+    int lane_rows = 0;               // longest segment
     bool lane = false;
     int2* rwork = nullptr; int nrwork = 0;
     int2* gwork = nullptr; int ngwork = 0; int gtile = 64;
@@ -190,7 +192,7 @@ template <class T> struct Batch : BatchBase {
     // counts of mhd2d_launch.h (with the 8% that a single grid asks of the march),
     // each instance's segments then of equal length; empty where the tiles are
     // faster, as for a batch of one wave of tiles.
-    std::vector<int2> lane_work() const {
+    std::vector<int2> lane_work(int& longest) const {
         std::vector<int2> w;
         if (sizeof(T) != 4) return w;
         auto div_up = [](long a, long b) { return (a + b - 1) / b; };
@@ -208,6 +210,7 @@ template <class T> struct Batch : BatchBase {
         if (rows == 0) return w;
         for (int i = 0; i < n; i++) {
             const int mine = (int)div_up(p[i].Ny, div_up(p[i].Ny, rows));
+            longest = std::max(longest, mine);
             for (long k = 0; k < ctas(i, mine); k++) w.push_back(make_int2(i, mine << 24 | (int)k));
         }
         return w;
@@ -375,7 +378,7 @@ template <class T> struct Batch : BatchBase {
             sgrid[k] = std::max(1, std::min(nswork[k], per_sm * nsm));
             sgrid[NS + k] = std::max(1, nswork[k]);
         }
-        const std::vector<int2> lw = lane_work();
+        const std::vector<int2> lw = lane_work(lane_rows);
         nlwork = (int)lw.size();
         lane = nlwork > 0;
         if (int r = upload_vec(&lwork, lw)) return r;
@@ -666,6 +669,8 @@ template <class T> struct Batch : BatchBase {
         return CC_OK;
     }
 
+    int march_candidate() const { return 2 * BatchLaunch<T>::n_shapes(); }
+
     int autotune(int reps, int* out_shape, double* out_ms) override {
         if (tc_fatal) return fail(h, CC_ERR_CUDA, "handle unusable: an earlier tensor-core transform gave up on its MMAs");
         if (!all_loaded()) return fail(h, CC_ERR_STATE, "not every instance has an uploaded state");
@@ -714,16 +719,18 @@ template <class T> struct Batch : BatchBase {
         if (best != shape || march != lane) invalidate_graph();
         shape = best;
         lane = march;
-        if (out_shape) *out_shape = best;
+        if (out_shape) *out_shape = lane ? march_candidate() : best;
         if (out_ms) *out_ms = best_ms;
         return CC_OK;
     }
 
     int set_shape(int k) override {
-        if (k < 0 || k >= 2 * BatchLaunch<T>::n_shapes()) return fail(h, CC_ERR_ARG, "no such stage candidate");
-        if (k != shape || lane) invalidate_graph();
-        shape = k;
-        lane = false;
+        if (k < 0 || k > march_candidate() || (k == march_candidate() && nlwork == 0))
+            return fail(h, CC_ERR_ARG, "no such stage candidate");
+        const bool march = k == march_candidate();
+        if (march != lane || (!march && k != shape)) invalidate_graph();
+        if (!march) shape = k;
+        lane = march;
         return CC_OK;
     }
 
@@ -732,13 +739,14 @@ template <class T> struct Batch : BatchBase {
         o->n = n;
         o->precision = sizeof(T) == 8 ? CC_FP64 : CC_FP32;
         for (int i = 0; i < n; i++) o->cells += (long long)p[i].Nx * p[i].Ny;
-        o->shape = shape;
         const int NS = BatchLaunch<T>::n_shapes();
-        o->n_shapes = 2 * NS;
+        o->shape = lane ? march_candidate() : shape;
+        o->n_shapes = march_candidate() + (nlwork > 0 ? 1 : 0);
         const TileShape sh = BatchLaunch<T>::shape(shape % NS);
-        o->tile_x = sh.tx; o->tile_y = sh.ty;
-        o->stage_tiles = nswork[shape % NS];
-        o->stage_ctas = sgrid[shape];
+        o->tile_x = lane ? LANE_W : sh.tx;
+        o->tile_y = lane ? lane_rows : sh.ty;
+        o->stage_tiles = lane ? nlwork : nswork[shape % NS];
+        o->stage_ctas = lane ? nlwork : sgrid[shape];
         o->reduce_tiles = nrwork;
         o->poisson_tiles = ngwork + ntcwork;
         o->poisson_tile = ntcwork > 0 ? (ngwork > 0 ? -128 : 128) : gtile;

@@ -38,10 +38,11 @@ typedef struct cc_batch_info {
     int32_t precision;       /* CC_FP64 or CC_FP32                         */
     int64_t cells;           /* sum of Nx*Ny over instances                */
     int32_t shape;           /* stage candidate in use                     */
-    int32_t n_shapes;        /* candidates: tile shapes x {persistent, one CTA per tile} */
-    int32_t tile_x, tile_y;  /* its tile                                   */
+    int32_t n_shapes;        /* candidates: tile shapes x {persistent, one CTA per tile}, and the register march
+                                where the batch has one                    */
+    int32_t tile_x, tile_y;  /* its tile (the march: columns of a strip, rows of the longest segment) */
     int32_t stage_tiles;     /* work-list length of the stage kernel       */
-    int32_t stage_ctas;      /* persistent CTAs of the stage kernel        */
+    int32_t stage_ctas;      /* CTAs of the stage kernel                   */
     int32_t reduce_tiles;    /* 32x8 reduce tiles (one partial each)       */
     int32_t poisson_tiles;   /* GEMM tiles of the direct solve             */
     int64_t device_bytes;    /* device memory held by the handle           */
@@ -76,8 +77,8 @@ int cc_batch_times(cc_handle* h, double* t);
  * stage time.  Candidate c uses tile shape c % S of the S compiled shapes,
  * launched persistent (c < S: one CTA per resident slot walking a contiguous
  * run of the tile work-list) or flat (c >= S: one CTA per tile).  An FP32 batch
- * of more than a wave of tiles runs its stages as warps that march in registers,
- * with the same bits, until a candidate is set or is found here to be faster. */
+ * of more than a wave of tiles has one more candidate, 2 S: its stages as warps
+ * that march in registers, with the same bits.  Such a batch starts with it. */
 int cc_batch_autotune(cc_handle* h, int reps, int* shape, double* ms);
 /* Use candidate `shape` (0 <= shape < n_shapes). */
 int cc_batch_set_shape(cc_handle* h, int shape);

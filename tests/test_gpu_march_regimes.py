@@ -90,7 +90,9 @@ def test_ensemble(regime, gravity):
     out = []
     for shape in (None, 0):
         with BatchSolver(params) as b:
-            if shape is not None:
+            if shape is None:
+                assert b.info()["shape"] == b.info()["n_shapes"] - 1   # the march
+            else:
                 b.set_shape(shape)
             for i, s in enumerate(states):
                 b.upload(i, *s)
