@@ -101,7 +101,7 @@ template <class T> struct Adjoint : AdjointBase, Batch<T> {
     bool loaded0 = false;
 
     Adjoint(cc_handle* hh, const cc_mhd2d_params& pp, int k, int mx)
-        : Batch<T>(hh, &pp, 1), K(k), max_steps(mx) {}
+        : Batch<T>(hh, &pp, 1), K(k), max_steps(mx) { this->down_late = true; }
 
     T* plane_alloc() {
         T* q = nullptr;

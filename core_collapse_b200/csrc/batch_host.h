@@ -147,8 +147,15 @@ template <class T> struct Batch : BatchBase {
     double* diag_part = nullptr;
     double* staging = nullptr;
     size_t staging_elems = 0;
-    static constexpr size_t DOWN_HALF = (size_t)4 << 20;   // bytes; pinned, two of them to a handle
+    // pageable downloads (down_buffers): two pinned halves and what is packed for one; down_half bytes, the
+    // largest instance's state or 4 MB.  From the set-up on (the pinned memory took 50 ms of a first
+    // download), but for a handle that has other ways to read its state (down_late: the adjoint's)
+    static constexpr size_t DOWN_HALF = (size_t)4 << 20;
+    bool down_late = false;
+    size_t down_half = 0;
+    bool down_tried = false;
     char* down = nullptr;
+    double* packed = nullptr;
     cudaEvent_t down_done[2] = {nullptr, nullptr};
     bool any_grav = false;
     int shape = 0;
@@ -232,6 +239,7 @@ template <class T> struct Batch : BatchBase {
             off[i] = total;
             total += (size_t)pitch[i] * (q.Ny + 1) * 25;
             staging_elems = std::max(staging_elems, (size_t)(q.Nx + 1) * (q.Ny + 1));
+            down_half = std::min(DOWN_HALF, std::max(down_half, sizeof(double) * 8 * (size_t)(q.Nx + 1) * (q.Ny + 1)));
             if (q.gravity_on) any_grav = true;
         }
         T* pool = nullptr;
@@ -392,11 +400,9 @@ template <class T> struct Batch : BatchBase {
         if (int r = dalloc(&active, n)) return r;
         if (int r = dalloc(&steps, n)) return r;
         if (int r = dalloc(&diag_part, (size_t)RED_BLOCKS * 7)) return r;
-        if (int r = dalloc(&staging, std::max(staging_elems, DOWN_HALF / sizeof(double)))) return r;
-        void* pin = nullptr;
-        if (cudaHostAlloc(&pin, 2 * DOWN_HALF, cudaHostAllocDefault) == cudaSuccess) down = static_cast<char*>(pin);
-        else cudaGetLastError();   // downloads then copy field by field
-        for (cudaEvent_t& e : down_done) CC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        if (int r = dalloc(&staging, staging_elems)) return r;
+        if (!down_late)
+            if (int r = down_buffers()) return r;
         CC_CUDA(cudaMemsetAsync(dt, 0, sizeof(double) * n, st()));
         CC_CUDA(cudaMemsetAsync(tclk, 0, sizeof(double) * n, st()));
         CC_CUDA(cudaMemsetAsync(rho_mean, 0, sizeof(double) * n, st()));
@@ -441,6 +447,24 @@ template <class T> struct Batch : BatchBase {
         return true;
     }
 
+    // the buffers of pageable downloads; where they cannot be had, packed stays null and fields are copied one by one
+    int down_buffers() {
+        if (down_tried) return CC_OK;
+        down_tried = true;
+        void *pin = nullptr, *dev = nullptr;
+        const size_t elems = std::max(staging_elems, down_half / sizeof(double));
+        if (cudaHostAlloc(&pin, 2 * down_half, cudaHostAllocDefault) == cudaSuccess) down = static_cast<char*>(pin);
+        if (down && cudaMalloc(&dev, sizeof(double) * elems) == cudaSuccess) allocs.push_back(dev);
+        if (!dev) {
+            cudaGetLastError();
+            return CC_OK;
+        }
+        for (cudaEvent_t& e : down_done) CC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        bytes += sizeof(double) * elems;
+        packed = static_cast<double*>(dev);
+        return CC_OK;
+    }
+
     int download(int i, double* const* f) override {
         if (i < 0 || i >= n || !f) return fail(h, CC_ERR_ARG, "bad instance index or null state");
         if (!loaded[i]) return fail(h, CC_ERR_STATE, "instance has no uploaded state");
@@ -448,7 +472,7 @@ template <class T> struct Batch : BatchBase {
         layout(i, w, hh);
         const Fields<T>& B = hinst[i].buf[cur];
         const T* src[8] = {B.rho, B.mx, B.my, B.mz, B.E, B.Bz, B.bx, B.by};
-        // Pageable destinations go through two pinned halves of DOWN_HALF bytes: as
+        // Pageable destinations go through two pinned halves of down_half bytes: as
         // many fields as fit are packed and copied by one transfer, and copied out of
         // one half while the next transfer fills the other (a larger field takes
         // pieces of its own).  Copied by itself into pageable memory, a field makes the
@@ -456,22 +480,24 @@ template <class T> struct Batch : BatchBase {
         // 135 ms into new arrays, and 96 this way (most of it their first touch).
         struct Part { int field; size_t src, off, bytes; };   // of a field, from byte src, to byte off of the half
         std::vector<std::vector<Part>> pieces;
-        size_t used = DOWN_HALF;                               // of the last piece
+        size_t used = down_half;                               // of the last piece
         for (int k = 0; k < 8; k++) {
             if (!f[k]) continue;
             const size_t all = sizeof(double) * (size_t)w[k] * hh[k];
             cudaPointerAttributes at{};
             const bool pageable = cudaPointerGetAttributes(&at, f[k]) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
             cudaGetLastError();
-            if (!pageable || !down) {
+            if (pageable)
+                if (int r = down_buffers()) return r;
+            if (!pageable || !packed) {
                 CC_CUDA(M2Launch<T>::pack_out(src[k], staging, w[k], hh[k], pitch[i], st()));
                 CC_CUDA(cudaMemcpyAsync(f[k], staging, all, cudaMemcpyDeviceToHost, st()));
                 h->perf.kernel_launches += 1;
-            } else if (all > DOWN_HALF) {
-                for (size_t b = 0; b < all; b += DOWN_HALF) pieces.push_back({Part{k, b, 0, std::min(all - b, DOWN_HALF)}});
-                used = DOWN_HALF;
+            } else if (all > down_half) {
+                for (size_t b = 0; b < all; b += down_half) pieces.push_back({Part{k, b, 0, std::min(all - b, down_half)}});
+                used = down_half;
             } else {
-                if (used + all > DOWN_HALF) { pieces.emplace_back(); used = 0; }
+                if (used + all > down_half) { pieces.emplace_back(); used = 0; }
                 pieces.back().push_back(Part{k, 0, used, all});
                 used += all;
             }
@@ -480,14 +506,14 @@ template <class T> struct Batch : BatchBase {
             size_t bytes = 0;
             for (const Part& x : pieces[q]) {
                 if (x.src == 0) {
-                    CC_CUDA(M2Launch<T>::pack_out(src[x.field], staging + x.off / sizeof(double), w[x.field], hh[x.field],
+                    CC_CUDA(M2Launch<T>::pack_out(src[x.field], packed + x.off / sizeof(double), w[x.field], hh[x.field],
                                                   pitch[i], st()));
                     h->perf.kernel_launches += 1;
                 }
                 bytes += x.bytes;
             }
-            const double* from = staging + pieces[q].front().src / sizeof(double);
-            CC_CUDA(cudaMemcpyAsync(down + (q & 1) * DOWN_HALF, from, bytes, cudaMemcpyDeviceToHost, st()));
+            const double* from = packed + pieces[q].front().src / sizeof(double);
+            CC_CUDA(cudaMemcpyAsync(down + (q & 1) * down_half, from, bytes, cudaMemcpyDeviceToHost, st()));
             CC_CUDA(cudaEventRecord(down_done[q & 1], st()));
             return CC_OK;
         };
@@ -498,7 +524,7 @@ template <class T> struct Batch : BatchBase {
                 if (int r = issue(q + 1)) return r;
             CC_CUDA(cudaEventSynchronize(down_done[q & 1]));
             for (const Part& x : pieces[q])
-                std::memcpy(reinterpret_cast<char*>(f[x.field]) + x.src, down + (q & 1) * DOWN_HALF + x.off, x.bytes);
+                std::memcpy(reinterpret_cast<char*>(f[x.field]) + x.src, down + (q & 1) * down_half + x.off, x.bytes);
         }
         CC_CUDA(cudaStreamSynchronize(st()));
         return CC_OK;
