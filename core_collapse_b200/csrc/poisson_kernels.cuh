@@ -312,6 +312,7 @@ struct SorArgs {
     int* iters_out;
     double* res_out;
     const int* active;
+    int max_polls = 1 << 26;   // of a wait of sor_cluster_kernel (a second or two), after which it gives up
 };
 
 // Lexicographic SOR, the reference's own solve (compute_poisson_gravity_periodic,
@@ -572,7 +573,7 @@ __global__ void __launch_bounds__(NT) sor_rb_kernel(SorArgs a) {
 //
 // Measured, per sweep, sor_rb_kernel -> this: 32^2 6.5 -> 1.6 us, 128^2 6.7 ->
 // 2.1, 256^2 8.3 -> 3.4, 350^2 9.6 -> 7.2; with the residual test at 50^2
-// 10.7 -> 2.8.  V = 8 is the last that gains: ten pairs a thread (400^2) took
+// 10.7 -> 2.9.  V = 8 is the last that gains: ten pairs a thread (400^2) took
 // 10.2 us against 10.1.
 //
 // 1024 consecutive pairs are a block of sor_rb_kernel; S is a multiple of
@@ -623,6 +624,7 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double s_val, s_res[SOR_CL_MAXC], s_max[NT / 32], s_over[2][SOR_CL_MAXC];
     __shared__ __align__(8) unsigned long long s_bar[6];   // red, black, parts x 2, over x 2
+    __shared__ int s_dead, s_any;                          // some thread's wait ran out; some residual is above tol
     const int nc = gridDim.x, c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nx = a.nx, ny = a.ny, half = (nx + 1) / 2, M = half * ny, W = S + 2 * half;
     const int k0 = c * S, k1 = (k0 + S < M) ? k0 + S : M;
@@ -634,10 +636,12 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
     const unsigned bars = smem_addr(s_bar), wins = smem_addr(win);
     enum { RED = 0, BLACK = 8, PARTS = 16, OVER = 32 };
     bool dead = false;
-    // wait for a phase of an mbarrier; bounded (about two seconds): a timeout is recorded and ends all further waits
+    // Wait for a phase of an mbarrier; bounded: a timeout is recorded, in s_dead too, and ends the thread's further
+    // waits.  The CTA must then not arrive again on a phase that is not complete: the next sweep expects nothing and
+    // ends where every thread has passed the barrier after the black cells and none can be waiting, so that all of
+    // them see the same s_dead.  The other CTAs run out of this one's values in turn.
     auto wait = [&](unsigned bar, unsigned parity) {
         if (dead) return;
-        long long t0 = 0;
         for (int polls = 0;; polls++) {
             unsigned ok = 0;
             asm volatile(
@@ -647,10 +651,7 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
                 : "r"(bars + bar), "r"(parity)
                 : "memory");
             if (ok) return;
-            if ((polls & 1023) == 1023) {
-                if (t0 == 0) t0 = clock64();
-                else if (clock64() - t0 > (4ll << 30)) { atomicExch(a.bar.err, 1); dead = true; return; }
-            }
+            if (polls >= a.max_polls) { atomicExch(a.bar.err, 1); s_dead = 1; dead = true; return; }
         }
     };
     auto expect = [&](unsigned bar, unsigned bytes) {
@@ -664,6 +665,7 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
     }
     const unsigned halo_bytes = 8u * halo, part_bytes = 8u * nb, over_bytes = 8u * nc;
     if (tid == 0) {
+        s_dead = 0;
         for (int b = 0; b < 6; b++)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bars + 8 * b) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -751,6 +753,7 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
     double m = 0.0;   // mean removal pending on every cell not yet rewritten in this sweep
     double res = 0.0;
     int it = 0;
+    bool gave_up = false;   // the same in every thread of a CTA
     // the neighbours W, E, N, S of the red (col 0) or black cell of pair v; `other`: the pair's other cell
     auto gather = [&](int v, int col, double other, double& pW, double& pE, double& pN, double& pS) {
         const unsigned y = col ? nbr[v].z : nbr[v].y;
@@ -800,10 +803,6 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
     };
     for (; it < a.max_iter; ++it) {
         const unsigned ph = it & 1, ph2 = (it >> 1) & 1, two = 8 * (it & 1);
-        if (tid == 0) {
-            if (nc > 1) { expect(RED, halo_bytes); expect(BLACK, halo_bytes); }
-            expect(PARTS + two, part_bytes);
-        }
         // Red: every value read is pending.  No branch but the rare ones, so that the V cells' chains
         // overlap.  A cell that does not exist (odd nx) takes the value that its neighbour, whose
         // clamped east it stands for, has there.
@@ -834,6 +833,10 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
         if (sends) {
 #pragma unroll
             for (int v = 0; v < V; v++) publish(v, 0, RED, vr[v]);
+        }
+        if (tid == 0 && !s_dead) {   // here rather than first: warp 0 is about to wait
+            if (nc > 1) { expect(RED, halo_bytes); expect(BLACK, halo_bytes); }
+            expect(PARTS + two, part_bytes);
         }
         if (edge) wait(RED, ph);
         __syncthreads();
@@ -885,7 +888,9 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
                 if (q4 == 0) usum[(u >> 5) * 33 + (u & 31)] = s;
             }
         }
+        const int stop = s_dead;   // written before the last barrier or behind the next one
         __syncthreads();
+        if (stop) { gave_up = true; break; }
         double* pt = parts + (it & 1) * nb;
         if (warp == 0) {
             const int v = lane >> 2, b = c * (S / 1024) + v;
@@ -908,17 +913,22 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
             const double r = residual();
             int any = __syncthreads_or(!(r < tol));
             if (nc > 1) {
-                if (tid == 0) expect(OVER + two, over_bytes);
-                if (tid < nc) store_counted(smem_addr(&s_over[it & 1][c]), bars + OVER + two, tid, any ? 1.0 : 0.0);
-                wait(OVER + two, ph2);
-                any = 0;
-                for (int q = 0; q < nc; q++) any |= s_over[it & 1][q] != 0.0;
+                if (warp == 0) {
+                    if (tid == 0) expect(OVER + two, over_bytes);
+                    if (lane < nc) store_counted(smem_addr(&s_over[it & 1][c]), bars + OVER + two, lane, any ? 1.0 : 0.0);
+                    wait(OVER + two, ph2);
+                    const double o = lane < nc ? s_over[it & 1][lane] : 0.0;
+                    any |= __any_sync(0xffffffffu, dead || o != 0.0);
+                    if (lane == 0) s_any = any;
+                }
+                __syncthreads();   // one warp waits and decides, so that every thread goes the same way
+                any = s_any;
             }
             if (!any || it + 1 == a.max_iter) res = cluster_max(r);
             if (!any) { ++it; break; }
         }
     }
-    if (!(tol > 0.0)) res = cluster_max(residual());
+    if (!(tol > 0.0) || gave_up) res = cluster_max(residual());   // once in every CTA, however it left the sweeps
 #pragma unroll
     for (int v = 0; v < V; v++) {
         const int k = k0 + v * NT + tid;
@@ -929,6 +939,8 @@ __global__ void __launch_bounds__(SOR_CL_NT, 1) sor_cluster_kernel(SorArgs a) {
     }
     if (c == 0 && tid == 0) { *a.iters_out = it; *a.res_out = res; }
     cl.sync();   // no CTA leaves while another may still store into its shared memory
+    if (s_dead)   // what was under way to it when a wait ran out
+        for (int k = 0; k < 100; k++) __nanosleep(1000);
 }
 
 // rhs = 4 pi G (rho - mean) (M2:187-194), mean from the density partial sums.
