@@ -100,3 +100,21 @@ def test_ensemble(regime, gravity):
             out.append([O.state_list(*b.download(i)) for i in range(len(params))])
     for i, (x, y) in enumerate(zip(*out)):
         _compare(x, y, f"{regime}, instance {i}")
+
+
+@pytest.mark.parametrize("regime", ("floors", "supersonic", "mixed"))
+def test_instance_without_gravity_beside_others_with_it(regime):
+    """Such an instance runs the stage kernel with gravity, alone it runs the one without."""
+    params = [_params(regime, 160, 144, gravity_on=i > 0, poisson="direct") for i in range(12)]
+    states = [_state(regime, p, 30 + i) for i, p in enumerate(params)]
+    out = []
+    for n, shape in ((12, None), (12, 0), (1, None)):
+        with BatchSolver(params[:n]) as b:
+            if shape is not None:
+                b.set_shape(shape)
+            for i in range(n):
+                b.upload(i, *states[i])
+            b.advance(3, np.zeros(n))
+            out.append(O.state_list(*b.download(0)))
+    _compare(out[0], out[2], regime)
+    _compare(out[1], out[2], regime)
