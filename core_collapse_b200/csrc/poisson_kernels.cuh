@@ -553,8 +553,8 @@ __global__ void __launch_bounds__(NT) sor_rb_kernel(SorArgs a) {
 // 256^2 for under 1 us of FP64 work.  Here the potential never leaves the SMs
 // and CTAs exchange single values (st.async into the other CTA's shared
 // memory, counted by an mbarrier there), so that no phase waits for a fence:
-// a cluster barrier of 1024 threads takes 700 cycles with its release fence,
-// a counted store to a neighbour 260, to all of 16 CTAs 490.
+// a cluster barrier of 1024 threads takes 680 cycles with its release fence, an
+// exchange by counted stores with a neighbour 380, with all of 16 CTAs 560.
 //
 // Cells go by pairs k = j half + p, the red and the black cell of columns 2p,
 // 2p + 1 of row j: N and S neighbours of either are the other colour's of
