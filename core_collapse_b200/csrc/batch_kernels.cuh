@@ -106,7 +106,7 @@ m2b_stage_kernel(const BatchInst<T>* __restrict__ inst, const int2* __restrict__
 // instance, a segment length and four (strip, segment) pairs of that instance,
 // one to a warp, so that instances of one or two strips fill their CTAs too.
 // The tiles' bits (Stage32).  128 square instances of 64 to 256 cells a side (164 on
-// average) with gravity, first / second stage: tiles 317 / 343 us -> 185 / 222.
+// average) with gravity, first / second stage: tiles 317 / 343 us -> 185 / 217.
 // The instance's constants and planes are copied out of shared memory first:
 // read there they are loaded again in every row (192 / 235 us).
 // ---------------------------------------------------------------------------

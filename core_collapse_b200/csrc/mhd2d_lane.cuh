@@ -20,7 +20,7 @@
 // Bound: issue (73% of the slots at 16 warps an SM; 128 registers allow no more,
 // and 20 warps at 96 registers spilled: 722 us) and the latency of a row's two
 // HLLD chains.  4096^2 with gravity, first / second stage of a step: tiles 1103
-// / 1156 us -> 661 / 778.  On the way: the potential carried instead of read at
+// / 1156 us -> 652 / 771.  On the way: the potential carried instead of read at
 // the update (717 -> 611 with the cheaper HLLD: a load there is waited for), the
 // state before the update kept in shared memory instead of read again and the
 // Joule sub-step from shuffles (864 -> 715, second stage).  1003 x 777: 51 / 54

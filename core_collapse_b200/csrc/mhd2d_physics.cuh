@@ -44,7 +44,7 @@ __host__ __device__ __forceinline__ Prim<T> prim_select(bool left, const Prim<T>
 // reference's quotients, each rounded as its division rounds it, but forms them
 // so that they overlap (Div in cc_device.cuh): the stage kernel is
 // bound by chains of dependent operations at 20 warps an SM, and the divisions
-// were the longest.  1024^2 stage kernel, second stage: 323 -> 255 us, RK
+// were the longest.  1024^2 stage kernel, second stage: 323 -> 258 us, RK
 // average 73 -> 55; 3D faces at 90 x 70 x 52 with the hybrid equation of state
 // 57 -> 50.  Sharing reciprocals alone, with a branch to each quotient, gained
 // nothing (328 us).
